@@ -15,6 +15,7 @@
 #include "bvh.h"
 #include "common.h"
 #include "lbvh.cuh"
+#include "radix_sort.cuh"
 #include "render_tree.cuh"
 #include "scene.h"
 #include "trace.cuh"
@@ -250,6 +251,12 @@ int upload_common(lg_renderer* r, const lg_scene_desc* d)
     return LG_OK;
 }
 
+// Scratch of build_wide_nodes and build_wide4_nodes for a render tree of n nodes.
+size_t record_scratch_bytes(int n)
+{
+    return ((size_t)n * 11 + 2 * ((size_t)n / 1024 + 1) + 256) * sizeof(int);
+}
+
 // Traversal records (2- and 4-wide) from the render tree tree_mode selects
 // (render_tree.cu): PLOC over the triangles, PLOC over the BuildBVH tree's
 // leaves, or that tree itself.
@@ -274,9 +281,7 @@ int build_records(lg_renderer* r)
     LG_TRY(rc);
     r->tree_used = mode;
     const int n = render_tree_nodes(nbvh, r->n_tris, mode);
-    const size_t nb = (size_t)n / 1024 + 1;
-    size_t need = ((size_t)n * 11 + 2 * nb + 256) * sizeof(int);
-    LG_TRY(r->scratch.reserve(need));
+    LG_TRY(r->scratch.reserve(record_scratch_bytes(n)));
     LG_TRY(r->wide4.reserve(((size_t)n / 2 + 1) * sizeof(Wide4Node)));
     int root = 0, ni = 0, nl = 0, root4 = 0, n4 = 0;
     LG_TRY_CUDA(build_wide_nodes(r->rnodes.as<lg_bvh_node>(), n, r->wide.as<WideNode>(), r->leaves.as<int2>(),
@@ -388,11 +393,14 @@ cudaError_t post_fault(lg_renderer* r, cudaStream_t st)
 // then the stream is drained first so no copy still in flight can set it again.
 int take_fault(lg_renderer* r)
 {
-    if (!*(volatile unsigned*)r->fault_host) return LG_OK;
+    const unsigned fault = *(volatile unsigned*)r->fault_host;
+    if (!fault) return LG_OK;
     LG_TRY_CUDA(cudaStreamSynchronize(r->stream));
     LG_TRY_CUDA(cudaMemsetAsync(r->fault.p, 0, sizeof(unsigned), r->stream));
     LG_TRY_CUDA(cudaStreamSynchronize(r->stream));
     *(volatile unsigned*)r->fault_host = 0u;
+    if (fault == kRadixSortError)
+        return set_error(LG_ERR_DEVICE, "a wait of the ray sort ran out: the image is not the sorted render's");
     return set_error(LG_ERR_DEVICE,
                      "traversal stack overflow: the BVH is deeper than the %d-entry traversal stack holds, so "
                      "some subtrees were skipped and the image is incomplete",
@@ -783,7 +791,7 @@ int lg_renderer_set_scene(lg_renderer* r, const lg_scene_desc* d)
         LG_TRY_CUDA(cudaMemcpyAsync(r->tris_in.p, d->tris, (size_t)n * sizeof(lg_triangle), cudaMemcpyHostToDevice,
                                     r->stream));
     LG_TRY(queue_material_check(r, r->tris_in.as<lg_triangle>(), n, d->n_mats));
-    LG_TRY(r->scratch.reserve(lbvh_scratch_bytes(n, false)));
+    LG_TRY(r->scratch.reserve(std::max(lbvh_scratch_bytes(n, false), record_scratch_bytes(std::max(2 * n, 1)))));
     int count = 0;
     LG_TRY(lbvh_build(r->tris_in.as<lg_triangle>(), n, r->nodes.as<lg_bvh_node>(), &count, nullptr,
                       r->tris.as<lg_triangle>(), r->scratch.p, r->scratch.bytes, r->stream));

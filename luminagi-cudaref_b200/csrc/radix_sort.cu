@@ -1,54 +1,64 @@
 // radix_sort.cu -- see radix_sort.cuh.
+//
+// Bound by latency at the sizes the library sorts (8 MB of pairs stay in L2): a
+// pass is one round of key loads, the ranking, the look-back and the writes.
+// One B200, 30-bit keys (4 passes): 59 us for 1,050,972 pairs and 21 us for
+// 20,500.  With three launches a pass (per-tile histogram, scan of the
+// [digit][tile] table, scatter with a block-wide sync per 256 keys) a pass took 30
+// and 20 us.
 #include "radix_sort.cuh"
 
 namespace lg
 {
 namespace
 {
-constexpr int kThreads = 256;
-constexpr int kItems = 16;  // keys per thread per tile
-constexpr int kTile = kThreads * kItems;
-constexpr int kWarps = kThreads / 32;
+constexpr int kHistThreads = 256;
 
-size_t tiles_for(size_t n) { return (n + kTile - 1) / kTile; }
+// Keys per tile.  A sort's tiles start together, so each looks back over many
+// unfinished ones: work that grows with the square of the tiles, 134 MB of reads a pass
+// at 1,050,972 keys in tiles of 2,048.  So the tiles grow with n to stay near one
+// per SM: 15 us a pass in tiles of 8,192 there, 22 us in tiles of 2,048.
+int tile_keys(size_t n) { return n <= 148 * 1024 ? 1024 : (n <= 148 * 2048 ? 2048 : (n <= 148 * 4096 ? 4096 : 8192)); }
+size_t tiles_for(size_t n) { return (n + tile_keys(n) - 1) / tile_keys(n); }
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-__global__ void __launch_bounds__(kThreads) hist_kernel(const uint32_t* __restrict__ keys, size_t n, int shift,
-                                                        int bits, uint32_t* __restrict__ counts, int tiles)
+// Digit totals of every pass in one read of the keys.
+__global__ void __launch_bounds__(kHistThreads) hist_kernel(const uint32_t* __restrict__ keys, size_t n, int begin_bit,
+                                                        int end_bit, uint32_t* __restrict__ hist)
 {
-    __shared__ uint32_t h[256];
-    for (int i = threadIdx.x; i < 256; i += kThreads) h[i] = 0;
+    __shared__ uint32_t h[kRadixMaxPasses][256];
+    for (int i = threadIdx.x; i < kRadixMaxPasses * 256; i += kHistThreads) (&h[0][0])[i] = 0;
     __syncthreads();
-    const size_t base = (size_t)blockIdx.x * kTile;
-    const uint32_t mask = (1u << bits) - 1u;
-#pragma unroll
-    for (int k = 0; k < kItems; ++k)
+    for (size_t i = (size_t)blockIdx.x * kHistThreads + threadIdx.x; i < n; i += (size_t)gridDim.x * kHistThreads)
     {
-        size_t i = base + (size_t)k * kThreads + threadIdx.x;
-        if (i < n) atomicAdd(&h[(keys[i] >> shift) & mask], 1u);
+        const uint32_t key = keys[i];
+        int p = 0;
+        for (int shift = begin_bit; shift < end_bit; shift += 8, ++p)
+        {
+            const int bits = min(8, end_bit - shift);
+            atomicAdd(&h[p][(key >> shift) & ((1u << bits) - 1u)], 1u);
+        }
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += kThreads) counts[(size_t)d * tiles + blockIdx.x] = h[d];
+    for (int i = threadIdx.x; i < kRadixMaxPasses * 256; i += kHistThreads)
+    {
+        const uint32_t c = (&h[0][0])[i];
+        if (c) atomicAdd(&hist[i], c);
+    }
 }
 
-// Exclusive scan of each digit's row of the [digit][tile] count table, one
-// block per digit (tiles is n / 4096, so a row is short), and the digit's
-// total.  The digits' own offsets (an exclusive scan of the 256 totals) are
-// added by every scatter block, so no single-block pass over the whole table
-// is needed.
-constexpr int kScanThreads = 256;
-__global__ void __launch_bounds__(kScanThreads) digit_scan_kernel(uint32_t* __restrict__ counts, int tiles,
-                                                                  uint32_t* __restrict__ digit_total)
+// A published count: two flag bits over the value.
+constexpr uint32_t kAggregate = 1u << 30;  // this tile's own count of the digit
+constexpr uint32_t kInclusive = 2u << 30;  // the count of all tiles up to this one
+constexpr uint32_t kValueMask = (1u << 30) - 1u;
+constexpr int kLookBack = 8;               // predecessors read at a time
+constexpr int kPollLimit = 1 << 22;        // polls of unpublished counts before a tile gives up
+
+// Exclusive scan over the first 256 threads of one value each (every thread of the block calls it).
+__device__ __forceinline__ uint32_t digit_excl(uint32_t v, uint32_t* warp_sums)
 {
-    __shared__ uint32_t warp_sums[kScanThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t* row = counts + (size_t)blockIdx.x * tiles;
-    const int per = (tiles + kScanThreads - 1) / kScanThreads;  // consecutive entries per thread
-    const int first = threadIdx.x * per;
-    uint32_t sum = 0;
-    for (int k = 0; k < per; ++k)
-        if (first + k < tiles) sum += row[first + k];
-    uint32_t x = sum;
+    uint32_t x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1)
     {
@@ -59,96 +69,168 @@ __global__ void __launch_bounds__(kScanThreads) digit_scan_kernel(uint32_t* __re
     __syncthreads();
     uint32_t before = 0;
     for (int w = 0; w < warp; ++w) before += warp_sums[w];
-    uint32_t run = before + x - sum;
-    for (int k = 0; k < per; ++k)
-        if (first + k < tiles)
-        {
-            const uint32_t v = row[first + k];
-            row[first + k] = run;
-            run += v;
-        }
-    if (threadIdx.x == kScanThreads - 1) digit_total[blockIdx.x] = run;
+    return before + x - v;
 }
 
-__global__ void __launch_bounds__(kThreads) scatter_kernel(const uint32_t* __restrict__ keys_in,
-                                                           const uint32_t* __restrict__ vals_in,
-                                                           uint32_t* __restrict__ keys_out,
-                                                           uint32_t* __restrict__ vals_out, size_t n, int shift,
-                                                           int bits, const uint32_t* __restrict__ offsets, int tiles,
-                                                           const uint32_t* __restrict__ digit_total)
+template <int kThreads, int kItems>
+struct PassShared
 {
-    __shared__ uint32_t digit_base[256];         // running position inside this tile
-    __shared__ uint32_t global_base[256];
-    __shared__ uint32_t warp_cnt[kWarps][256];   // per-round counts, then exclusive prefix across warps
-    __shared__ uint32_t round_total[256];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    static constexpr int kWarps = kThreads / 32;
+    uint32_t warp_cnt[kWarps][256];  // per-warp digit counts, then their exclusive prefix across warps
+    uint32_t tile_start[256];        // first place of the digit within the tile
+    uint32_t global_base[256];       // global place of the digit's first key, less tile_start
+    uint32_t sums[2][kWarps];
+    uint32_t tile, pad[3];
+    uint32_t key[kThreads * kItems], val[kThreads * kItems];
+};
+
+template <int kThreads, int kItems, bool kIota>
+__global__ void __launch_bounds__(kThreads) pass_kernel(const uint32_t* __restrict__ keys_in,
+                                                        const uint32_t* __restrict__ vals_in,
+                                                        uint32_t* __restrict__ keys_out,
+                                                        uint32_t* __restrict__ vals_out, uint32_t n, int shift,
+                                                        int bits, const uint32_t* __restrict__ hist, uint32_t* state,
+                                                        uint32_t* ticket, uint32_t* error)
+{
+    constexpr int kTile = kThreads * kItems, kWarps = kThreads / 32;
+    static_assert(kThreads >= 256, "one digit per thread");
+    extern __shared__ __align__(16) unsigned char pass_mem[];
+    PassShared<kThreads, kItems>& sh = *reinterpret_cast<PassShared<kThreads, kItems>*>(pass_mem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) sh.tile = atomicAdd(ticket, 1u);
+    for (int i = tid; i < kWarps * 256; i += kThreads) (&sh.warp_cnt[0][0])[i] = 0;
+    const uint32_t digit_total = tid < 256 ? hist[tid] : 0u;
+    __syncthreads();
+    const uint32_t tile = sh.tile;
     const uint32_t mask = (1u << bits) - 1u;
-    // Digit offsets: exclusive scan of the 256 digit totals (one per thread).
-    static_assert(kThreads == 256, "one digit per thread");
-    {
-        const uint32_t t = digit_total[threadIdx.x];
-        uint32_t x = t;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) round_total[warp] = x;
-        __syncthreads();
-        uint32_t before = 0;
-        for (int w = 0; w < warp; ++w) before += round_total[w];
-        digit_base[threadIdx.x] = 0;
-        global_base[threadIdx.x] = before + x - t + offsets[(size_t)threadIdx.x * tiles + blockIdx.x];
-        __syncthreads();
-    }
-    const size_t base = (size_t)blockIdx.x * kTile;
+    const uint32_t base = tile * (uint32_t)kTile;
+    const uint32_t count = min((uint32_t)kTile, n - base);
     const uint32_t lt_mask = (1u << lane) - 1u;
+
+    // Keys in (warp, item, lane) order, so a warp ranks its own run of 32 * kItems keys without a block sync.
+    uint32_t key[kItems], val[kItems], rank[kItems];
+#pragma unroll
     for (int k = 0; k < kItems; ++k)
     {
-        for (int d = threadIdx.x; d < 256 * kWarps; d += kThreads) (&warp_cnt[0][0])[d] = 0;
-        __syncthreads();
-        const size_t i = base + (size_t)k * kThreads + threadIdx.x;
-        const bool valid = i < n;
-        uint32_t key = valid ? keys_in[i] : 0u;
-        uint32_t val = valid ? vals_in[i] : 0u;
-        // Invalid lanes get digit 256 so they never match a real digit.
-        uint32_t digit = valid ? ((key >> shift) & mask) : 256u;
-        uint32_t peers = __match_any_sync(0xffffffffu, digit);
-        uint32_t rank_in_warp = __popc(peers & lt_mask);
-        if (valid && rank_in_warp == 0) warp_cnt[warp][digit] = __popc(peers);
-        __syncthreads();
-        // Exclusive prefix across warps, one digit per thread.
-        for (int d = threadIdx.x; d < 256; d += kThreads)
-        {
-            uint32_t run = 0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w)
-            {
-                uint32_t c = warp_cnt[w][d];
-                warp_cnt[w][d] = run;
-                run += c;
-            }
-            round_total[d] = run;
-        }
-        __syncthreads();
-        if (valid)
-        {
-            uint32_t pos = global_base[digit] + digit_base[digit] + warp_cnt[warp][digit] + rank_in_warp;
-            keys_out[pos] = key;
-            vals_out[pos] = val;
-        }
-        __syncthreads();
-        for (int d = threadIdx.x; d < 256; d += kThreads) digit_base[d] += round_total[d];
-        __syncthreads();
+        const uint32_t i = (uint32_t)(warp * kItems + k) * 32u + lane;
+        key[k] = i < count ? keys_in[base + i] : 0u;
+        val[k] = kIota ? base + i : (i < count ? vals_in[base + i] : 0u);
     }
+#pragma unroll
+    for (int k = 0; k < kItems; ++k)
+    {
+        const uint32_t i = (uint32_t)(warp * kItems + k) * 32u + lane;
+        const bool valid = i < count;
+        // keys past the end get digit 256, which matches no real one
+        const uint32_t digit = valid ? ((key[k] >> shift) & mask) : 256u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, digit);
+        const uint32_t before = valid ? sh.warp_cnt[warp][digit] : 0u;
+        __syncwarp();
+        if (valid && (peers & lt_mask) == 0) sh.warp_cnt[warp][digit] = before + __popc(peers);
+        __syncwarp();
+        rank[k] = before + __popc(peers & lt_mask);
+    }
+    __syncthreads();
+
+    // One digit per thread: the tile's count, published for the tiles after it.
+    uint32_t total = 0;
+    volatile uint32_t* mine = state + (size_t)tile * 256 + tid;
+    if (tid < 256)
+    {
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w)
+        {
+            const uint32_t c = sh.warp_cnt[w][tid];
+            sh.warp_cnt[w][tid] = total;
+            total += c;
+        }
+        *mine = (tile == 0 ? kInclusive : kAggregate) | total;
+    }
+    const uint32_t start = digit_excl(total, sh.sums[0]);
+    const uint32_t digit_base = digit_excl(digit_total, sh.sums[1]);
+    if (tid < 256)
+    {
+        uint32_t before = 0;
+        if (tile > 0)
+        {
+            // Add up the counts of the tiles before, nearest first, until one has its inclusive count.
+            int j = (int)tile - 1, polls = 0;
+            bool done = false;
+            while (!done)
+            {
+                uint32_t v[kLookBack];
+#pragma unroll
+                for (int b = 0; b < kLookBack; ++b)
+                    v[b] = j - b >= 0 ? *(volatile uint32_t*)(state + (size_t)(j - b) * 256 + tid) : 0u;
+#pragma unroll
+                for (int b = 0; b < kLookBack; ++b)
+                {
+                    if (done || j < 0 || (v[b] >> 30) == 0) break;
+                    before += v[b] & kValueMask;
+                    if (v[b] >> 30 == 2) done = true;
+                    --j;
+                }
+                if (!done && ++polls > kPollLimit)
+                {
+                    *error = kRadixSortError;
+                    break;
+                }
+            }
+            *mine = kInclusive | ((before + total) & kValueMask);
+        }
+        sh.tile_start[tid] = start;
+        sh.global_base[tid] = digit_base + before - start;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kItems; ++k)
+    {
+        const uint32_t i = (uint32_t)(warp * kItems + k) * 32u + lane;
+        if (i >= count) continue;
+        const uint32_t digit = (key[k] >> shift) & mask;
+        const uint32_t at = sh.tile_start[digit] + sh.warp_cnt[warp][digit] + rank[k];
+        sh.key[at] = key[k];
+        sh.val[at] = val[k];
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < count; i += kThreads)
+    {
+        const uint32_t k = sh.key[i];
+        const uint32_t pos = sh.global_base[(k >> shift) & mask] + i;
+        if (pos < n)  // always, unless a wait ran out
+        {
+            keys_out[pos] = k;
+            vals_out[pos] = sh.val[i];
+        }
+    }
+}
+
+struct PassArgs
+{
+    const uint32_t *ki, *vi;
+    uint32_t *ko, *vo;
+    uint32_t n;
+    int shift, bits;
+    const uint32_t* hist;
+    uint32_t *state, *ticket, *error;
+};
+template <int kThreads, int kItems>
+cudaError_t launch_pass(const PassArgs& a, bool iota, size_t tiles, cudaStream_t st)
+{
+    const int smem = (int)sizeof(PassShared<kThreads, kItems>);
+    auto k = iota ? pass_kernel<kThreads, kItems, true> : pass_kernel<kThreads, kItems, false>;
+    const cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k<<<(unsigned)tiles, kThreads, smem, st>>>(a.ki, a.vi, a.ko, a.vo, a.n, a.shift, a.bits, a.hist, a.state, a.ticket,
+                                               a.error);
+    return cudaGetLastError();
 }
 }  // namespace
 
 size_t radix_sort_scratch_bytes(size_t n)
 {
-    size_t t = tiles_for(n ? n : 1);
-    return align256(n * 4) * 2 + align256(256 * t * 4) + 256 * 4 + 256;
+    const size_t t = tiles_for(n ? n : 1);
+    return align256(n * 4) * 2 + align256(kRadixMaxPasses * 256 * 4 + 64) + kRadixMaxPasses * t * 256 * 4 + 512;
 }
 
 RadixSortScratch radix_sort_bind(void* base, size_t n)
@@ -159,31 +241,55 @@ RadixSortScratch radix_sort_bind(void* base, size_t n)
     p += align256(n * 4);
     s.vals_alt = (uint32_t*)p;
     p += align256(n * 4);
-    s.counts = (uint32_t*)p;
-    p += align256(256 * tiles_for(n ? n : 1) * 4);
-    s.digit_total = (uint32_t*)p;
+    s.hist = (uint32_t*)p;
+    s.tickets = s.hist + kRadixMaxPasses * 256;
+    s.error = s.tickets + kRadixMaxPasses;
+    p += align256(kRadixMaxPasses * 256 * 4 + 64);
+    s.state = (uint32_t*)p;
+    s.zero_bytes = (size_t)((char*)(s.state + kRadixMaxPasses * tiles_for(n ? n : 1) * 256) - (char*)s.hist);
     s.capacity = n;
     return s;
 }
 
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
-                             const RadixSortScratch& s, cudaStream_t stream)
+                             const RadixSortScratch& s, cudaStream_t stream, bool counted, bool iota)
 {
-    if (n <= 1 || end_bit <= begin_bit) return cudaSuccess;
-    const int tiles = (int)tiles_for(n);
+    if (!counted)
+    {
+        const cudaError_t e = cudaMemsetAsync(s.hist, 0, s.zero_bytes, stream);
+        if (e != cudaSuccess) return e;
+    }
+    if (n <= 1 || end_bit <= begin_bit)
+        return iota && n == 1 ? cudaMemsetAsync(vals, 0, 4, stream) : cudaSuccess;
+    if (n >= (1ull << 30) || end_bit - begin_bit > 8 * kRadixMaxPasses) return cudaErrorInvalidValue;
+    const size_t tiles = tiles_for(n);
+    cudaError_t e = cudaSuccess;
+    if (!counted)
+    {
+        const size_t blocks = (n + kHistThreads * 4 - 1) / (kHistThreads * 4);
+        hist_kernel<<<(unsigned)(blocks < 592 ? blocks : 592), kHistThreads, 0, stream>>>(keys, n, begin_bit, end_bit,
+                                                                                        s.hist);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     uint32_t *ki = keys, *vi = vals, *ko = s.keys_alt, *vo = s.vals_alt;
-    for (int shift = begin_bit; shift < end_bit; shift += 8)
+    int pass = 0;
+    for (int shift = begin_bit; shift < end_bit; shift += 8, ++pass)
     {
         const int bits = (end_bit - shift) < 8 ? (end_bit - shift) : 8;
-        hist_kernel<<<tiles, kThreads, 0, stream>>>(ki, n, shift, bits, s.counts, tiles);
-        digit_scan_kernel<<<256, kScanThreads, 0, stream>>>(s.counts, tiles, s.digit_total);
-        scatter_kernel<<<tiles, kThreads, 0, stream>>>(ki, vi, ko, vo, n, shift, bits, s.counts, tiles,
-                                                       s.digit_total);
+        const PassArgs a{ki, vi, ko, vo, (uint32_t)n, shift, bits, s.hist + pass * 256,
+                         s.state + (size_t)pass * tiles * 256, s.tickets + pass, s.error};
+        const bool first = iota && pass == 0;
+        switch (tile_keys(n))
+        {
+            case 1024: e = launch_pass<256, 4>(a, first, tiles, stream); break;
+            case 2048: e = launch_pass<256, 8>(a, first, tiles, stream); break;
+            case 4096: e = launch_pass<512, 8>(a, first, tiles, stream); break;
+            default: e = launch_pass<512, 16>(a, first, tiles, stream); break;
+        }
+        if (e != cudaSuccess) return e;
         uint32_t* t = ki; ki = ko; ko = t;
         t = vi; vi = vo; vo = t;
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
     if (ki != keys)
     {
         e = cudaMemcpyAsync(keys, ki, n * 4, cudaMemcpyDeviceToDevice, stream);

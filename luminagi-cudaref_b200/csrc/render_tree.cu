@@ -493,13 +493,16 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
     parent_of_kernel<<<g, kTB, 0, st>>>(src, n_nodes, parent);
     depth_of_kernel<<<g, kTB, 0, st>>>(n_nodes, root, parent, depth, ids);
     LG_TRY_CUDA(cudaGetLastError());
-    LG_TRY_CUDA(radix_sort_pairs(depth, ids, (size_t)n_nodes, 0, 8, radix_sort_bind(sort_mem, (size_t)n_nodes), st));
-    uint32_t max_depth = 0;
+    const RadixSortScratch rs = radix_sort_bind(sort_mem, (size_t)n_nodes);
+    LG_TRY_CUDA(radix_sort_pairs(depth, ids, (size_t)n_nodes, 0, 8, rs, st));
+    uint32_t max_depth = 0, sort_error = 0;
+    LG_TRY_CUDA(cudaMemcpyAsync(&sort_error, rs.error, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     LG_TRY_CUDA(cudaMemcpyAsync(&max_depth, depth + n_nodes - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     rank_kernel<<<g, kTB, 0, st>>>(ids, n_nodes, newpos);
     emit_kernel<<<g, kTB, 0, st>>>(src, ids, newpos, n_nodes, d_out);
     LG_TRY_CUDA(cudaGetLastError());
     LG_TRY_CUDA(cudaStreamSynchronize(st));
+    if (sort_error) return set_error(LG_ERR_DEVICE, "render tree: a wait of the sort ran out");
     if (max_depth >= 255u) return set_error(LG_ERR_CAPACITY, "render tree: depth over 254");
     return LG_OK;
 }
