@@ -474,11 +474,14 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) trace_kernel(D
     Counters cnt{0, 0, 0, 0, 0, 0};
     PathState st;
     Trav q;
-    int stack[kStack];
+    int stack_mem[kStack + 1];
+    const Stack stack(stack_mem);
     const int root = kWidth == 4 ? s.root4 : s.root;
     const int thresh = job.refill_threshold < 1 ? 1 : (job.refill_threshold > 32 ? 32 : job.refill_threshold);
     const int quorum = job.leaf_quorum < 0 ? 0 : (job.leaf_quorum > 31 ? 31 : job.leaf_quorum);
-    bool active = false, exhausted = false, tdone = false;
+    bool active = false, exhausted = false;
+    q.cur = kDone;
+    q.pend = 0;
     for (;;)
     {
         // Refill idle lanes with one atomic per warp.
@@ -524,8 +527,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) trace_kernel(D
                         st.k = 0;
                         st.pixel = (unsigned)((st.py * c.width + st.px) * 3);
                         start_sample(st, c);
-                        trav_begin<kCount>(q, root, st.tmax, st.li >= 0, cnt);
-                        tdone = false;
+                        trav_begin<kCount>(q, stack, root, st.tmax, st.li >= 0, cnt);
                         active = true;
                     }
                 }
@@ -535,23 +537,16 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) trace_kernel(D
         // Lanes that stay idle for good (work exhausted) do not count towards
         // the threshold; idle lanes that can still be refilled do.
         const int idle_final = exhausted ? __popc(__ballot_sync(0xffffffffu, !active)) : 0;
-        for (;;)
-        {
-            if (warp_step<kWidth, kCount, kWT, kChecked>(s, st.ray, st.li >= 0, active && !tdone, quorum, q, stack,
-                                                         cnt, s_top, top_n))
-                tdone = true;
-            const unsigned busy = __ballot_sync(0xffffffffu, active && !tdone);
-            if (busy == 0 || 32 - __popc(busy) - idle_final >= thresh) break;
-        }
-        if (active && tdone)
+        trav_run<kWidth, kCount, kWT, kChecked>(s, st.ray, st.li >= 0, quorum, thresh, idle_final, q, stack, cnt, s_top,
+                                                top_n);
+        if (active && q.cur == kDone && q.pend == 0)
         {
             const DevCam& c = kBatch ? job.jobs[st.job].cam : cam;
             // batched: the frame's bounce limit is read from the job table (one register less than keeping it)
             const int max_b = kBatch ? job.jobs[st.job].max_bounces : job.max_bounces;
             if (advance<kAcc64>(st, s, c, max_b, q.tri, q.t, q.u, q.v))
             {
-                trav_begin<kCount>(q, root, st.tmax, st.li >= 0, cnt);
-                tdone = false;
+                trav_begin<kCount>(q, stack, root, st.tmax, st.li >= 0, cnt);
             }
             else
             {

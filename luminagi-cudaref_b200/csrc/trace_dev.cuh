@@ -68,18 +68,19 @@ __device__ __forceinline__ bool tri_hit(const Ray& r, const float4* __restrict__
     const vec3 v0 = v3(a.x, a.y, a.z);
     const vec3 e1 = v3(b.x, b.y, b.z);
     const vec3 e2 = v3(c.x, c.y, c.z);
+    // every value first, then one decision: in a warp some lane nearly always needs all of them, and an early
+    // return is a divergent branch
     vec3 p = cross(r.d, e2);
     float det = dot(e1, p);
-    if (det > -kEps && det < kEps) return false;
     float invDet = 1.0f / det;
     vec3 s = vsub(r.o, v0);
     float u = dot(s, p) * invDet;
-    if (u < 0.0f || u > 1.0f) return false;
     vec3 q = cross(s, e1);
     float v = dot(r.d, q) * invDet;
-    if (v < 0.0f || u + v > 1.0f) return false;
     float tt = dot(e2, q) * invDet;
-    if (tt <= kEps || tt >= tmax) return false;
+    const bool miss = (det > -kEps && det < kEps) | (u < 0.0f) | (u > 1.0f) | (v < 0.0f) | (u + v > 1.0f) |
+                      (tt <= kEps) | (tt >= tmax);
+    if (miss) return false;
     outT = tt;
     outU = u;
     outV = v;
@@ -163,21 +164,57 @@ __device__ __forceinline__ void cswap(float& ta, int& la, float& tb, int& lb)
 
 // Traversal state of one ray: the record or leaf link to visit next (kDone
 // once the stack is empty), a leaf postponed for testing (0 = none; leaf
-// links are negative), the stack depth, and the closest hit so far (t starts
-// at the ray's tmax).
-constexpr int kDone = (int)0x80000000;  // no leaf or record link takes this value
+// links are negative), the stack's next free entry, and the closest hit so far
+// (t starts at the ray's tmax).  The stack's entry 0 holds kDone, so popping
+// needs no test for an empty stack.
+constexpr int kDone = (int)0x80000000;  // no deeper link takes this value; every leaf link is above it as unsigned
 struct Trav
 {
-    int cur, pend, sp, tri;
+    int cur, pend, tri;
+    unsigned sp;
     float t, u, v;
 };
 
-template <bool kCount>
-__device__ __forceinline__ void trav_begin(Trav& q, int root, float tmax, bool anyhit, Counters& cnt)
+// A ray's stack: one int per entry in local memory, addressed in bytes from
+// its base.  push_if / pop_if are predicated instructions, not branches: a
+// visit has four of them, and the step loop as a whole had 30 branches.  With
+// this, one vote less per step and the triangle test without early returns,
+// the 8-spp engine frame (1728x864, 2 bounces, 65.4 M rays) went from 36.65 to
+// 34.5 ms, the 32-spp box frame from 9.9 to 9.3 ms; same images.
+struct Stack
 {
-    q.cur = root;
-    q.pend = 0;
-    q.sp = 0;
+    unsigned base;  // local address
+    __device__ __forceinline__ explicit Stack(int* m)
+    {
+        base = (unsigned)__cvta_generic_to_local(m);
+        asm volatile("st.local.u32 [%0], %1;" ::"r"(base), "r"(kDone) : "memory");
+    }
+    __device__ __forceinline__ unsigned first() const { return base + 4u; }
+    __device__ __forceinline__ void push_if(bool p, unsigned& sp, int v) const
+    {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p st.local.u32 [%0], %1;\n\t@p add.u32 %0, %0, 4;\n\t}"
+            : "+r"(sp)
+            : "r"(v), "r"((int)p)
+            : "memory");
+    }
+    __device__ __forceinline__ void pop_if(bool p, unsigned& sp, int& v) const
+    {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p sub.u32 %0, %0, 4;\n\t@p ld.local.u32 %1, [%0];\n\t}"
+            : "+r"(sp), "+r"(v)
+            : "r"((int)p)
+            : "memory");
+    }
+};
+
+template <bool kCount>
+__device__ __forceinline__ void trav_begin(Trav& q, const Stack& st, int root, float tmax, bool anyhit, Counters& cnt)
+{
+    // a root that is a leaf is held like any other
+    q.cur = root >= 0 ? root : kDone;
+    q.pend = root >= 0 ? 0 : root;
+    q.sp = st.first();
     q.tri = -1;
     q.t = tmax;
     q.u = 0.0f;
@@ -185,28 +222,30 @@ __device__ __forceinline__ void trav_begin(Trav& q, int root, float tmax, bool a
     if (kCount) { if (anyhit) cnt.shadow++; else cnt.closest++; }
 }
 
-__device__ __forceinline__ int pop(Trav& q, const int* stack) { return q.sp == 0 ? kDone : stack[--q.sp]; }
-
-// Stacks `link`; a push past kStack entries is dropped and flags the scene's
-// fault word (the host turns it into LG_ERR_DEVICE), so a tree too deep for
-// the stack never yields a silently incomplete image.  kChecked = false is
-// for trees whose stack bound (computed when their records are built) fits
-// in kStack: no traversal over them can overflow, so the test is left out.
+// Stacks `link` if p; a push past kStack entries is dropped and flags the
+// scene's fault word (the host turns it into LG_ERR_DEVICE), so a tree too
+// deep for the stack never yields a silently incomplete image.  kChecked =
+// false is for trees whose stack bound (computed when their records are
+// built) fits in kStack: no traversal over them can overflow, so the test is
+// left out.
 template <bool kCount, bool kChecked = true>
-__device__ __forceinline__ void push(Trav& q, int* stack, int link, const DevScene& s, Counters& cnt)
+__device__ __forceinline__ void push(bool p, Trav& q, const Stack& st, int link, const DevScene& s, Counters& cnt)
 {
-    if (!kChecked)
+    if (kChecked && p && q.sp >= st.first() + 4u * kStack)
     {
-        stack[q.sp++] = link;
-        return;
+        if (kCount) cnt.overflow++;
+        *s.fault = 1u;
+        p = false;
     }
-    if (q.sp < kStack)
-    {
-        stack[q.sp++] = link;
-        return;
-    }
-    if (kCount) cnt.overflow++;
-    *s.fault = 1u;
+    st.push_if(p, q.sp, link);
+}
+
+// A lane that has reached a leaf and holds none takes it and goes on with its stack.
+__device__ __forceinline__ void hold_leaf(Trav& q, const Stack& st)
+{
+    const bool p = q.pend == 0 && (unsigned)q.cur > (unsigned)kDone;
+    q.pend = p ? q.cur : q.pend;
+    st.pop_if(p, q.sp, q.cur);
 }
 
 // The four boxes of a quantized 4-wide record against one ray.  Per axis,
@@ -278,14 +317,14 @@ __device__ __forceinline__ int4 box4(const float (&a)[8], const float (&b)[8], c
 // rest are stacked nearest-on-top.  2-wide (traverse_closest, :109-160, for
 // one record): both children's boxes with the reference's slab arithmetic,
 // the nearer hit child first and the farther one stacked.  With no child hit
-// the next entry is popped (kDone when the stack is empty).
+// the next entry is popped (kDone at the bottom of the stack).
 // Measured alternatives on the 64-spp engine frame (633 ms with whole-ray
 // traversal and records from the even-depth collapse): a "while-while" loop
 // without speculation (internal records until every lane holds a leaf, then
 // the leaves) ran 745 ms, and a 24-entry shared-memory stack 675 ms (its
 // 96 KB per SM comes out of the L1 that caches the BVH records).
 template <int kWidth, bool kCount, bool kChecked = true>
-__device__ __forceinline__ void node_step(const DevScene& s, const Ray& r, Trav& q, int* stack, Counters& cnt,
+__device__ __forceinline__ void node_step(const DevScene& s, const Ray& r, Trav& q, const Stack& st, Counters& cnt,
                                           const Wide4Node* s_top = nullptr, int top_n = 0)
 {
     if (kCount) cnt.nodes++;
@@ -302,15 +341,12 @@ __device__ __forceinline__ void node_step(const DevScene& s, const Ray& r, Trav&
         cswap(t0, l0, t2, l2);
         cswap(t1, l1, t3, l3);
         cswap(t1, l1, t2, l2);
-        if (t0 != inf)
-        {
-            // push farthest first so the nearest remaining is on top
-            if (t3 != inf) push<kCount, kChecked>(q, stack, l3, s, cnt);
-            if (t2 != inf) push<kCount, kChecked>(q, stack, l2, s, cnt);
-            if (t1 != inf) push<kCount, kChecked>(q, stack, l1, s, cnt);
-            q.cur = l0;
-            return;
-        }
+        // farthest first, so the nearest remaining is on top
+        push<kCount, kChecked>(t3 != inf, q, st, l3, s, cnt);
+        push<kCount, kChecked>(t2 != inf, q, st, l2, s, cnt);
+        push<kCount, kChecked>(t1 != inf, q, st, l1, s, cnt);
+        q.cur = l0;
+        st.pop_if(t0 == inf, q.sp, q.cur);
     }
     else
     {
@@ -321,20 +357,11 @@ __device__ __forceinline__ void node_step(const DevScene& s, const Ray& r, Trav&
         float t0, t1;
         const bool h0 = slab(r, xy0.x, xy0.y, xy0.z, xy0.w, z01.x, z01.y, q.t, t0);
         const bool h1 = slab(r, xy1.x, xy1.y, xy1.z, xy1.w, z01.z, z01.w, q.t, t1);
-        if (h0 && h1)
-        {
-            const bool swap = t1 < t0;
-            push<kCount, kChecked>(q, stack, swap ? ln.x : ln.y, s, cnt);
-            q.cur = swap ? ln.y : ln.x;
-            return;
-        }
-        if (h0 || h1)
-        {
-            q.cur = h0 ? ln.x : ln.y;
-            return;
-        }
+        const bool second = h1 && (!h0 || t1 < t0);  // child 1 is entered first
+        push<kCount, kChecked>(h0 && h1, q, st, second ? ln.x : ln.y, s, cnt);
+        q.cur = second ? ln.y : ln.x;
+        st.pop_if(!h0 && !h1, q.sp, q.cur);
     }
-    q.cur = pop(q, stack);
 }
 
 // Tests every triangle of leaf `link` in order (strict < on t, as
@@ -385,17 +412,19 @@ template <int kWidth, bool kCount, bool kWT>
 __device__ __forceinline__ int traverse_ray(const DevScene& s, const Ray& r, float tmax, bool anyhit, float& bestT,
                                             float& bestU, float& bestV, Counters& cnt)
 {
-    int stack[kStack];
+    int stack[kStack + 1];
+    const Stack st(stack);
     Trav q;
-    trav_begin<kCount>(q, kWidth == 4 ? s.root4 : s.root, tmax, anyhit, cnt);
-    while (q.cur != kDone)
+    trav_begin<kCount>(q, st, kWidth == 4 ? s.root4 : s.root, tmax, anyhit, cnt);
+    while (q.cur != kDone || q.pend != 0)
     {
-        if (q.cur >= 0) node_step<kWidth, kCount>(s, r, q, stack, cnt);
-        else
+        if (q.pend != 0)
         {
-            if (leaf_step<kWidth, kCount, kWT>(s, r, anyhit, q.cur, q, cnt)) break;
-            q.cur = pop(q, stack);
+            if (leaf_step<kWidth, kCount, kWT>(s, r, anyhit, q.pend, q, cnt)) break;
+            q.pend = 0;
         }
+        else node_step<kWidth, kCount>(s, r, q, st, cnt);
+        hold_leaf(q, st);
     }
     bestT = q.t;
     bestU = q.u;
@@ -403,41 +432,45 @@ __device__ __forceinline__ int traverse_ray(const DevScene& s, const Ray& r, flo
     return q.tri;
 }
 
-// One warp-wide step of the persistent kernel's traversals, with leaves
-// postponed (Aila and Laine, "Understanding the Efficiency of Ray Traversal
-// on GPUs", HPG 2009): a lane that reaches a leaf sets it aside and keeps
-// visiting records from its stack while other lanes still look for a leaf.
-// The warp visits records while more than `quorum` lanes are still looking
-// (or no lane holds a leaf), and otherwise tests the held leaves together;
-// quorum 0 waits for every lane, as in the paper.  Every step makes
-// progress: a record step has at least one searching lane, a leaf step at
-// least one held leaf.  The records visited past a postponed leaf would be
-// culled by a nearer hit in it only for closest-hit rays, and then only cost
-// time: the closest hit is the same (up to exact ties in t).  `busy` is this
-// lane's ray in flight; returns true when its traversal has finished.
+// Steps a warp's traversals until `thresh` lanes more than `idle_final` have
+// none left in flight (or all have), with leaves postponed (Aila and Laine,
+// "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009): a lane
+// that reaches a leaf sets it aside and keeps visiting records from its stack
+// while other lanes still look for a leaf.  The warp visits records while
+// more than `quorum` lanes are still looking (or no lane holds a leaf), and
+// otherwise tests the held leaves together; quorum 0 waits for every lane, as
+// in the paper.  Every step makes progress: a record step has at least one
+// searching lane, a leaf step at least one held leaf.  The records visited
+// past a postponed leaf would be culled by a nearer hit in it only for
+// closest-hit rays, and then only cost time: the closest hit is the same (up
+// to exact ties in t).  A lane without a ray in flight has cur == kDone and
+// pend == 0.
 template <int kWidth, bool kCount, bool kWT, bool kChecked = true>
-__device__ __forceinline__ bool warp_step(const DevScene& s, const Ray& r, bool anyhit, bool busy, int quorum,
-                                          Trav& q, int* stack, Counters& cnt, const Wide4Node* s_top, int top_n)
+__device__ __forceinline__ void trav_run(const DevScene& s, const Ray& r, bool anyhit, int quorum, int thresh,
+                                         int idle_final, Trav& q, const Stack& st, Counters& cnt,
+                                         const Wide4Node* s_top, int top_n)
 {
-    if (busy && q.pend == 0 && q.cur < 0 && q.cur != kDone)
+    for (;;)
     {
-        q.pend = q.cur;
-        q.cur = pop(q, stack);
+        const unsigned busy = __ballot_sync(0xffffffffu, q.cur != kDone || q.pend != 0);
+        if (busy == 0 || 32 - __popc(busy) - idle_final >= thresh) return;
+        const unsigned searching = __ballot_sync(0xffffffffu, q.pend == 0 && q.cur >= 0);
+        if (__popc(searching) > quorum || searching == busy)
+        {
+            if (q.cur >= 0)
+            {
+                node_step<kWidth, kCount, kChecked>(s, r, q, st, cnt, s_top, top_n);
+                hold_leaf(q, st);
+            }
+        }
+        else if (q.pend != 0)
+        {
+            const bool stop = leaf_step<kWidth, kCount, kWT>(s, r, anyhit, q.pend, q, cnt);
+            q.pend = 0;
+            if (stop) q.cur = kDone;
+            hold_leaf(q, st);
+        }
     }
-    const bool fin = busy && q.pend == 0 && q.cur == kDone;
-    // every lane takes part in the votes, finished or idle ones included
-    const bool searching = busy && !fin && q.pend == 0;  // then q.cur >= 0
-    const unsigned n_searching = __popc(__ballot_sync(0xffffffffu, searching));
-    const bool holding = __any_sync(0xffffffffu, busy && !fin && q.pend != 0);
-    if (n_searching > (unsigned)quorum || !holding)
-    {
-        if (busy && q.cur >= 0) node_step<kWidth, kCount, kChecked>(s, r, q, stack, cnt, s_top, top_n);
-        return fin;
-    }
-    if (!busy || fin || q.pend == 0) return fin;
-    const int link = q.pend;
-    q.pend = 0;
-    return leaf_step<kWidth, kCount, kWT>(s, r, anyhit, link, q, cnt) || q.cur == kDone;
 }
 
 // xorshift32 / randf (pathtracer.cu:193-204).

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kWfThreads) wf_bounce_kernel(DevScene s, int n
 // expressions in the same order, so the image does not change (up to rays
 // whose two nearest triangles tie exactly); the traversals become
 // persistent warps that step their lanes through traversals one record or
-// leaf at a time (warp_step, leaves postponed) and take the next ray of
+// leaf at a time (trav_run, leaves postponed) and take the next ray of
 // the list as soon as enough lanes are free, with no shading in between.
 constexpr int kWfListThreads = 256;
 // The staged bounce keeps a shadow ray, a contribution and a flag per (light, ray): 52 bytes per light and pixel.
@@ -255,8 +255,11 @@ __global__ void __launch_bounds__(kWfListThreads, 4)
     const unsigned lt_mask = (1u << lane) - 1u;
     const int root = kWidth == 4 ? s.root4 : s.root;
     Counters cnt{0, 0, 0, 0, 0, 0};
-    int stack[kStack];
+    int stack_mem[kStack + 1];
+    const Stack stack(stack_mem);
     Trav q;
+    q.cur = kDone;
+    q.pend = 0;
     Ray ray;
     float tmax = 0.0f;
     int idx = -1;
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(kWfListThreads, 4)
                     idx = (int)i;
                     if (list_ray<kAny>(rays_in, order, so, sd, idx, ray, tmax))
                     {
-                        trav_begin<false>(q, root, tmax, kAny, cnt);
+                        trav_begin<false>(q, stack, root, tmax, kAny, cnt);
                         active = true;
                     }
                     else if (kAny) occ[idx] = 0;  // a skipped light: nothing traced
@@ -292,8 +295,9 @@ __global__ void __launch_bounds__(kWfListThreads, 4)
             if (exhausted) break;
             continue;
         }
-        if (warp_step<kWidth, false, kWT, kChecked>(s, ray, kAny, active, quorum, q, stack, cnt, nullptr, 0) &&
-            active)
+        const int idle_final = exhausted ? __popc(__ballot_sync(0xffffffffu, !active)) : 0;
+        trav_run<kWidth, false, kWT, kChecked>(s, ray, kAny, quorum, thresh, idle_final, q, stack, cnt, nullptr, 0);
+        if (active && q.cur == kDone && q.pend == 0)
         {
             if (kAny) occ[idx] = q.tri >= 0 ? 1 : 0;
             else hit[idx] = make_int4(q.tri, __float_as_int(q.t), __float_as_int(q.u), __float_as_int(q.v));
