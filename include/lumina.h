@@ -339,6 +339,12 @@ int lg_unet_get_params(lg_unet* u, float* params, int64_t n);
 int lg_unet_forward(lg_unet* u, const float* x, int n, int h, int w, float* y);
 /* Same on device buffers, ordered on `stream` (a cudaStream_t; NULL = synchronous). */
 int lg_unet_forward_device(lg_unet* u, const float* d_x, int n, int h, int w, float* d_y, void* stream);
+/* The denoiser on an 8-bit image (tools/denoise.py:34-52): images[k] are
+ * in_ch / 3 host frames of h*w*3 bytes (colour; with 12 channels also albedo,
+ * normal and position), u8/255, replicate-padded to multiples of 8; the
+ * network's output cropped, (u8)(clip(y,0,1)*255 + 0.5) into out (h*w*3
+ * bytes, host).  in_ch must be a multiple of 3. */
+int lg_unet_denoise_rgb8(lg_unet* u, const uint8_t* const* images, int h, int w, uint8_t* out);
 /* Training (reference ml/train.py:184-201): mean L1 loss of the network output
  * against target, backward pass on the tensor cores, and one Adam step
  * (betas 0.9/0.999, eps 1e-8, bias correction, as torch.optim.Adam) on the

@@ -67,6 +67,32 @@ __global__ void f32_tonemap_kernel(const float* __restrict__ in, long long HW, u
     }
 }
 
+// u8 / 255 of the frame's pixels, the last row and column repeated out to hp x wp; grid (ceil(hp*wp / 256), frames).
+__global__ void pad_rgb8_kernel(const uint8_t* __restrict__ in, int h, int w, float* __restrict__ out, int hp, int wp)
+{
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x, HW = (long long)hp * wp;
+    if (p >= HW) return;
+    const int y = (int)(p / wp), x = (int)(p % wp);
+    const uint8_t* s = in + (((size_t)blockIdx.y * h + min(y, h - 1)) * w + min(x, w - 1)) * 3;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) out[((long long)blockIdx.y * 3 + c) * HW + p] = (float)s[c] / 255.0f;
+}
+
+// The first h rows and w columns of an hp x wp image as 8-bit pixels, product and sum rounded one by one (as the
+// host's clip(v,0,1)*255 + 0.5, tools/denoise.py:51).
+__global__ void crop_rgb8_kernel(const float* __restrict__ in, int hp, int wp, uint8_t* __restrict__ out, int h, int w)
+{
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= (long long)h * w) return;
+    const long long at = p / w * wp + p % w;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+    {
+        const float v = fminf(fmaxf(in[c * (long long)hp * wp + at], 0.0f), 1.0f);
+        out[p * 3 + c] = (uint8_t)__fadd_rn(__fmul_rn(v, 255.0f), 0.5f);
+    }
+}
+
 // Grid of the per-pixel conversions.
 dim3 px_grid(long long HW, int n) { return dim3((unsigned)((HW + 255) / 256), (unsigned)n); }
 
@@ -89,6 +115,20 @@ __global__ void gather_kernel(const float* __restrict__ imgs, int H, int W, cons
     out[i] = imgs[(((long long)cr.img * 3 + c) * H + cr.y + yy) * W + cr.x + xx];
 }
 }  // namespace
+
+namespace lg
+{
+cudaError_t pad_rgb8(const uint8_t* d_in, int frames, int h, int w, float* d_out, int hp, int wp, cudaStream_t st)
+{
+    pad_rgb8_kernel<<<px_grid((long long)hp * wp, frames), 256, 0, st>>>(d_in, h, w, d_out, hp, wp);
+    return cudaGetLastError();
+}
+cudaError_t crop_rgb8(const float* d_in, int hp, int wp, uint8_t* d_out, int h, int w, cudaStream_t st)
+{
+    crop_rgb8_kernel<<<px_grid((long long)h * w, 1), 256, 0, st>>>(d_in, hp, wp, d_out, h, w);
+    return cudaGetLastError();
+}
+}  // namespace lg
 
 extern "C" {
 

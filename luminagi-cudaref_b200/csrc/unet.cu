@@ -292,7 +292,7 @@ void lg_unet_destroy(lg_unet* u)
     u->params.release();
     for (auto& b : u->packed) b.release();
     for (Buf* b : {&u->x0, &u->t1, &u->cat1, &u->p1, &u->t2, &u->cat2, &u->p2, &u->t3, &u->cat3, &u->p3, &u->t4,
-                   &u->t5, &u->t6, &u->t7, &u->u1, &u->xin, &u->yout, &u->err, &u->grads, &u->adam_m, &u->adam_v,
+                   &u->t5, &u->t6, &u->t7, &u->u1, &u->xin, &u->yout, &u->img8, &u->err, &u->grads, &u->adam_m, &u->adam_v,
                    &u->loss, &u->gs1, &u->gs2, &u->gs3, &u->tgt, &u->lo7, &u->lo9, &u->lo11, &u->gup, &u->wpart, &u->bpart, &u->tpart,
                    &u->uh1, &u->uh2, &u->uh3})
         b->release();
@@ -389,6 +389,32 @@ int lg_unet_forward(lg_unet* u, const float* x, int n, int h, int w, float* y)
     LG_TRY_CUDA(cudaStreamSynchronize(u->stream));
     int err = 0;
     LG_TRY_CUDA(cudaMemcpy(&err, u->err.p, sizeof(int), cudaMemcpyDeviceToHost));
+    if (err) return set_error(LG_ERR_DEVICE, "convolution kernel reported wait timeout %d", err);
+    return LG_OK;
+}
+
+int lg_unet_denoise_rgb8(lg_unet* u, const uint8_t* const* images, int h, int w, uint8_t* out)
+{
+    if (!u || !images || !out) return set_error(LG_ERR_INVALID, "NULL argument");
+    if (h <= 0 || w <= 0 || u->in_ch % 3)
+        return set_error(LG_ERR_INVALID, "denoise_rgb8: %dx%d image, %d input channels", h, w, u->in_ch);
+    const int frames = u->in_ch / 3, hp = (h + 7) / 8 * 8, wp = (w + 7) / 8 * 8;
+    for (int k = 0; k < frames; ++k)
+        if (!images[k]) return set_error(LG_ERR_INVALID, "NULL image %d", k);
+    const size_t frame = (size_t)h * w * 3, plane = (size_t)hp * wp;
+    LG_TRY(u->img8.ensure(frame * frames));
+    LG_TRY(u->xin.ensure(plane * u->in_ch * sizeof(float)));
+    LG_TRY(u->yout.ensure(plane * 3 * sizeof(float)));
+    uint8_t* img = (uint8_t*)u->img8.p;
+    for (int k = 0; k < frames; ++k)
+        LG_TRY_CUDA(cudaMemcpyAsync(img + k * frame, images[k], frame, cudaMemcpyHostToDevice, u->stream));
+    LG_TRY_CUDA(pad_rgb8(img, frames, h, w, (float*)u->xin.p, hp, wp, u->stream));
+    LG_TRY(forward_device_impl(u, (const float*)u->xin.p, 1, hp, wp, (float*)u->yout.p, false));
+    LG_TRY_CUDA(crop_rgb8((const float*)u->yout.p, hp, wp, img, h, w, u->stream));
+    int err = 0;
+    LG_TRY_CUDA(cudaMemcpyAsync(&err, u->err.p, sizeof(int), cudaMemcpyDeviceToHost, u->stream));
+    LG_TRY_CUDA(cudaMemcpyAsync(out, img, frame, cudaMemcpyDeviceToHost, u->stream));
+    LG_TRY_CUDA(cudaStreamSynchronize(u->stream));
     if (err) return set_error(LG_ERR_DEVICE, "convolution kernel reported wait timeout %d", err);
     return LG_OK;
 }

