@@ -21,6 +21,13 @@ __device__ __forceinline__ uint64_t global_timer_ns()
     return t;
 }
 
+// Programmatic dependent launch: let the next kernel of the stream start its
+// blocks as soon as this grid's have all started, and wait until the kernels
+// before this one have finished and their writes are visible (a no-op in a
+// launch without the attribute).
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

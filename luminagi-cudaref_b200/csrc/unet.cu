@@ -155,8 +155,7 @@ int forward_device_impl(lg_unet* u, const float* d_x, int N, int H, int W, float
     LG_TRY(pack_all_impl(u));
     LG_TRY(ensure_acts(u, N, H, W));
     cudaStream_t st = u->stream;
-    LG_TRY_CUDA(cudaMemsetAsync(u->err.p, 0, sizeof(int), st));
-    LG_TRY_CUDA(to_blocked_bf16(d_x, N, u->in_ch, H, W, (bf*)u->x0.p, 16, st, u->log_hdr, true));
+    LG_TRY_CUDA(to_blocked_bf16(d_x, N, u->in_ch, H, W, (bf*)u->x0.p, 16, st, u->log_hdr, true, (int*)u->err.p));
     const int H2 = H / 2, W2 = W / 2, H4 = H / 4, W4 = W / 4, H8 = H / 8, W8 = W / 8;
     // inference with nearest upsampling: u3a, u2a, u1a fold their upsampled inputs where their tiles allow
     const bool fold = !keep_u1;
@@ -189,7 +188,7 @@ int forward_device_impl(lg_unet* u, const float* d_x, int N, int H, int W, float
         }
         const bool probe = layer == u->probe_layer;
         if (probe) LG_TRY_CUDA(cudaEventRecord(u->probe_ev0, st));
-        LG_TRY_CUDA(conv3x3_forward((const bf*)in, a, st));
+        LG_TRY_CUDA(conv3x3_forward((const bf*)in, a, st, &u->plan[layer]));
         if (probe) LG_TRY_CUDA(cudaEventRecord(u->probe_ev1, st));
         return LG_OK;
     };
@@ -338,20 +337,15 @@ int lg_unet_forward_device(lg_unet* u, const float* d_x, int n, int h, int w, fl
     if (!u || !d_x || !d_y) return set_error(LG_ERR_INVALID, "NULL argument");
     if (stream)
     {
-        cudaEvent_t ev;
-        LG_TRY_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        cudaEventRecord(ev, (cudaStream_t)stream);
-        cudaStreamWaitEvent(u->stream, ev, 0);
-        cudaEventDestroy(ev);
+        if (!u->order_ev) LG_TRY_CUDA(cudaEventCreateWithFlags(&u->order_ev, cudaEventDisableTiming));
+        LG_TRY_CUDA(cudaEventRecord(u->order_ev, (cudaStream_t)stream));
+        LG_TRY_CUDA(cudaStreamWaitEvent(u->stream, u->order_ev, 0));
     }
     LG_TRY(forward_device_impl(u, d_x, n, h, w, d_y, false));
     if (stream)
     {
-        cudaEvent_t ev;
-        LG_TRY_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        cudaEventRecord(ev, u->stream);
-        cudaStreamWaitEvent((cudaStream_t)stream, ev, 0);
-        cudaEventDestroy(ev);
+        LG_TRY_CUDA(cudaEventRecord(u->order_ev, u->stream));
+        LG_TRY_CUDA(cudaStreamWaitEvent((cudaStream_t)stream, u->order_ev, 0));
         return LG_OK;
     }
     LG_TRY_CUDA(cudaStreamSynchronize(u->stream));

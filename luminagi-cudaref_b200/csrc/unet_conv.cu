@@ -18,7 +18,9 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
 #include <mutex>
+#include <utility>
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -423,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
     __shared__ EpiConsts ec;
 
     const int tid = threadIdx.x, warp = tid >> 5;
-    stage_epi_consts(a, ec, tid, kThreads);  // visible after the __syncthreads below
+    tc::launch_dependents();
     const int n_cot = a.Cout / BN;
     const int x0 = blockIdx.x * kTileX;
     const int y0 = blockIdx.y * kRows;
@@ -435,11 +437,6 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
     constexpr uint32_t kLboA = kHaloY * kHaloX * 16;
     constexpr uint32_t kLboB = BN * 16;
 
-    if (warp == 0)
-    {
-        tc::tmem_alloc(tmem_slot, kCols);
-        tc::tmem_relinquish();
-    }
     if (tid == 0)
     {
         s_fail = 0;
@@ -450,6 +447,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
         }
         tc::mbar_init(done, 1);
         tc::fence_mbar_init();
+    }
+    tc::wait_for_predecessors();
+    stage_epi_consts(a, ec, tid, kThreads);  // visible after the __syncthreads below
+    if (warp == 0)
+    {
+        tc::tmem_alloc(tmem_slot, kCols);
+        tc::tmem_relinquish();
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -617,7 +621,7 @@ __global__ void __launch_bounds__(kPThreads, 1) conv3x3_tc_persistent(const __gr
     __shared__ EpiConsts ec;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    stage_epi_consts(a, ec, tid, kPThreads);  // visible after the __syncthreads below
+    tc::launch_dependents();
     const int n_cot = a.Cout / BN;
     const int tiles_x = (a.W + kTileX - 1) / kTileX, tiles_y = (a.H + ROWS - 1) / ROWS;
     const int n_tiles = tiles_x * tiles_y * a.N * n_cot;
@@ -650,11 +654,6 @@ __global__ void __launch_bounds__(kPThreads, 1) conv3x3_tc_persistent(const __gr
         if (a.err) atomicExch(a.err, code);
     };
 
-    if (warp == 1)
-    {
-        tc::tmem_alloc(tmem_slot, kCols);
-        tc::tmem_relinquish();
-    }
     if (tid == 0)
     {
         s_fail = 0;
@@ -671,6 +670,15 @@ __global__ void __launch_bounds__(kPThreads, 1) conv3x3_tc_persistent(const __gr
         tc::mbar_init(done, 1);
         tc::mbar_init(wfull, 1);
         tc::fence_mbar_init();
+    }
+    // Nothing above reads or writes device memory, and TMEM is taken only here: a block that waits for the kernel
+    // before it holds nothing that kernel's blocks could need.
+    tc::wait_for_predecessors();
+    stage_epi_consts(a, ec, tid, kPThreads);  // visible after the __syncthreads below
+    if (warp == 1)
+    {
+        tc::tmem_alloc(tmem_slot, kCols);
+        tc::tmem_relinquish();
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -959,74 +967,104 @@ cudaError_t make_map_chunked(CUtensorMap* m, const __nv_bfloat16* base, int N, i
 // for the kernel's static shared memory (the epilogue constants, 1.4 KB).
 constexpr int kMaxSmem = 225 * 1024;
 
-template <int BN, int KC, int STAGES, bool RESW = false, int ROWS = kRows, bool DYP = false, bool VUP = false>
-cudaError_t launch_persistent(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream)
+// A launch whose blocks may start while the previous kernel of the stream is still running; every kernel
+// launched so waits (wait_for_predecessors) before it touches device memory.
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*fn)(P...), dim3 grid, int block, int smem, cudaStream_t stream, A&&... args)
 {
-    const int KB = a.Cin / KC;
-    if (RESW && a.Cout != BN) return cudaErrorInvalidValue;  // one output block only
-    if (VUP != (a.up_C > 0)) return cudaErrorInvalidValue;
-    // folded upsampling: both parts whole K-blocks, at least one skip K-block first, even rows
-    if (VUP && (!a.up_h || a.up_C % KC || a.Cin - a.up_C < KC || (a.H & 1))) return cudaErrorInvalidValue;
-    const int smem = PSmem<BN, KC, RESW, ROWS, DYP ? kChunkX : kHaloX>::bytes(STAGES, KB);
-    if (smem > kMaxSmem) return cudaErrorInvalidValue;
-    CUtensorMap m, m2;
-    ConvArgs b = a;
-    b.a_chunked = DYP && a.W % 8 == 0;
-    cudaError_t e = !DYP ? make_map(&m, in, a.N, a.Cin, a.H, a.W, KC, ROWS + 2)
-                    : b.a_chunked ? make_map_chunked(&m, in, a.N, a.Cin, a.H, a.W, KC, ROWS + 2)
-                                  : make_map(&m, in, a.N, a.Cin, a.H, a.W, KC, ROWS + 2, kChunkX);
-    if (e != cudaSuccess) return e;
-    m2 = m;
-    if (VUP)
-    {
-        e = b.a_chunked ? make_map_chunked(&m2, a.up_h, a.N, a.up_C, a.H / 2, a.W, KC, ROWS / 2 + 2)
-                        : make_map(&m2, a.up_h, a.N, a.up_C, a.H / 2, a.W, KC, ROWS / 2 + 2, kChunkX);
-        if (e != cudaSuccess) return e;
-    }
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = (size_t)smem;
+    c.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, fn, std::forward<A>(args)...);
+}
+
+template <int BN, int KC, int STAGES, bool RESW = false, int ROWS = kRows, bool DYP = false, bool VUP = false>
+cudaError_t launch_persistent(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan& plan)
+{
     auto fn = conv3x3_tc_persistent<BN, KC, STAGES, RESW, ROWS, DYP, VUP>;
-    // The resident-weights form's smem depends on KB: size the attribute for
-    // the largest launch it may see and query occupancy per launch size.
-    static bool attr_done = false;
-    static int sm_count = 0;
-    if (!attr_done)
+    if (!plan.ready)
     {
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+        const int KB = a.Cin / KC;
+        if (RESW && a.Cout != BN) return cudaErrorInvalidValue;  // one output block only
+        if (VUP != (a.up_C > 0)) return cudaErrorInvalidValue;
+        // folded upsampling: both parts whole K-blocks, at least one skip K-block first, even rows
+        if (VUP && (!a.up_h || a.up_C % KC || a.Cin - a.up_C < KC || (a.H & 1))) return cudaErrorInvalidValue;
+        const int smem = PSmem<BN, KC, RESW, ROWS, DYP ? kChunkX : kHaloX>::bytes(STAGES, KB);
+        if (smem > kMaxSmem) return cudaErrorInvalidValue;
+        plan.smem = smem;
+        plan.a_chunked = DYP && a.W % 8 == 0;
+        cudaError_t e = !DYP ? make_map(&plan.m, in, a.N, a.Cin, a.H, a.W, KC, ROWS + 2)
+                        : plan.a_chunked ? make_map_chunked(&plan.m, in, a.N, a.Cin, a.H, a.W, KC, ROWS + 2)
+                                         : make_map(&plan.m, in, a.N, a.Cin, a.H, a.W, KC, ROWS + 2, kChunkX);
         if (e != cudaSuccess) return e;
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-        attr_done = true;
+        plan.m2 = plan.m;
+        if (VUP)
+        {
+            e = plan.a_chunked ? make_map_chunked(&plan.m2, a.up_h, a.N, a.up_C, a.H / 2, a.W, KC, ROWS / 2 + 2)
+                               : make_map(&plan.m2, a.up_h, a.N, a.up_C, a.H / 2, a.W, KC, ROWS / 2 + 2, kChunkX);
+            if (e != cudaSuccess) return e;
+        }
+        // The resident-weights form's smem depends on KB: size the attribute for
+        // the largest launch it may see and query occupancy per launch size.
+        static bool attr_done = false;
+        static int sm_count = 0;
+        if (!attr_done)
+        {
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+            if (e != cudaSuccess) return e;
+            int dev = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+            attr_done = true;
+        }
+        int per_sm = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPThreads, smem);
+        if (e != cudaSuccess) return e;
+        // TMEM: each CTA holds 2*ROWS*BN of the SM's 512 columns for its lifetime
+        const int tmem_fit = 512 / (2 * ROWS * BN);
+        if (per_sm > tmem_fit) per_sm = tmem_fit;
+        if (per_sm < 1) per_sm = 1;
+        const long long tiles =
+            (long long)((a.W + kTileX - 1) / kTileX) * ((a.H + ROWS - 1) / ROWS) * a.N * (a.Cout / BN);
+        plan.grid[0] = (unsigned)std::min<long long>(tiles, (long long)per_sm * sm_count);
+        plan.grid[1] = plan.grid[2] = 1;
+        plan.ready = true;
     }
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPThreads, smem);
-    if (e != cudaSuccess) return e;
-    // TMEM: each CTA holds 2*ROWS*BN of the SM's 512 columns for its lifetime
-    const int tmem_fit = 512 / (2 * ROWS * BN);
-    if (per_sm > tmem_fit) per_sm = tmem_fit;
-    if (per_sm < 1) per_sm = 1;
-    const long long tiles = (long long)((a.W + kTileX - 1) / kTileX) * ((a.H + ROWS - 1) / ROWS) * a.N * (a.Cout / BN);
-    const long long grid = std::min<long long>(tiles, (long long)per_sm * sm_count);
-    fn<<<(unsigned)grid, kPThreads, smem, stream>>>(m, m2, b);
-    return cudaGetLastError();
+    ConvArgs b = a;
+    b.a_chunked = plan.a_chunked;
+    return launch_dependent(fn, dim3(plan.grid[0]), kPThreads, plan.smem, stream, plan.m, plan.m2, b);
 }
 
 template <int BN, int KC, int STAGES>
-cudaError_t launch(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream)
+cudaError_t launch(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan& plan)
 {
-    CUtensorMap m;
-    cudaError_t e = make_map(&m, in, a.N, a.Cin, a.H, a.W, KC);
-    if (e != cudaSuccess) return e;
-    const int smem = STAGES * Smem<BN, KC>::kStage + 1024 + 256;
-    static bool attr_done = false;
-    if (!attr_done)
+    if (!plan.ready)
     {
-        e = cudaFuncSetAttribute(conv3x3_tc_kernel<BN, KC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = make_map(&plan.m, in, a.N, a.Cin, a.H, a.W, KC);
         if (e != cudaSuccess) return e;
-        attr_done = true;
+        plan.smem = STAGES * Smem<BN, KC>::kStage + 1024 + 256;
+        static bool attr_done = false;
+        if (!attr_done)
+        {
+            e = cudaFuncSetAttribute(conv3x3_tc_kernel<BN, KC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     plan.smem);
+            if (e != cudaSuccess) return e;
+            attr_done = true;
+        }
+        plan.grid[0] = (unsigned)((a.W + kTileX - 1) / kTileX);
+        plan.grid[1] = (unsigned)((a.H + kRows - 1) / kRows);
+        plan.grid[2] = (unsigned)(a.N * (a.Cout / BN));
+        plan.ready = true;
     }
-    dim3 grid((a.W + kTileX - 1) / kTileX, (a.H + kRows - 1) / kRows, a.N * (a.Cout / BN));
-    conv3x3_tc_kernel<BN, KC, STAGES><<<grid, kThreads, smem, stream>>>(m, a);
-    return cudaGetLastError();
+    return launch_dependent(conv3x3_tc_kernel<BN, KC, STAGES>, dim3(plan.grid[0], plan.grid[1], plan.grid[2]), kThreads,
+                            plan.smem, stream, plan.m, a);
 }
 
 // Position i of a packed weight array -> (ct, kb, tap, kc8, j, e): output
@@ -1157,9 +1195,10 @@ __global__ void pack_folded_kernel(const float* __restrict__ w, int Cout, int Ci
 // reads the block's channels from their NCHW planes (consecutive threads,
 // consecutive pixels of a plane) and writes the pixel's 16 bytes.
 __global__ void to_blocked_kernel(const float* __restrict__ x, int N, int C, int H, int W,
-                                  __nv_bfloat16* __restrict__ out, int Cpad, int nb, int log1p_in)
+                                  __nv_bfloat16* __restrict__ out, int Cpad, int nb, int log1p_in, int* clear)
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // over N * nb * H * W
+    if (clear && i == 0) *clear = 0;
     const size_t HW = (size_t)H * W;
     if (i >= (size_t)N * nb * HW) return;
     const size_t p = i % HW;
@@ -1324,7 +1363,7 @@ cudaError_t conv_pack_many(const ConvPackJob* jobs, int n, cudaStream_t stream)
 }
 
 
-cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream)
+cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan* kept)
 {
     if (a.Cin % 16 != 0 || (a.Cout != 32 && a.Cout != 64 && a.Cout != 128 && a.Cout != 256)) return cudaErrorInvalidValue;
     if (a.epilogue == kEpiTail && a.Cout != 32) return cudaErrorInvalidValue;
@@ -1336,96 +1375,114 @@ cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStre
     const TileCfg c = resolve(a.tile, a.Cin, a.Cout);
     if (a.Cout % c.bn || a.Cin % c.kc) return cudaErrorInvalidValue;
     const int key = c.bn * 1000 + c.kc * 10 + c.stages;
+    ConvPlan once;
+    ConvPlan& plan = kept ? *kept : once;
+    ConvPlan::Key k;
+    std::memset(&k, 0, sizeof k);
+    k.in = in;
+    k.up_h = a.up_h;
+    k.N = a.N;
+    k.H = a.H;
+    k.W = a.W;
+    k.Cin = a.Cin;
+    k.Cout = a.Cout;
+    k.up_C = a.up_C;
+    k.tile = c;
+    if (std::memcmp(&k, &plan.key, sizeof k) != 0)
+    {
+        plan.ready = false;
+        std::memcpy(&plan.key, &k, sizeof k);
+    }
     if (a.up_C > 0)
     {
         if (!conv_tile_folds(c, a.Cin, a.Cout, a.up_C)) return cudaErrorInvalidValue;
-        if (c.persist == 7) return launch_persistent<32, 32, 2, false, 8, true, true>(in, a, stream);
-        if (key == 64322) return launch_persistent<64, 32, 2, false, 4, true, true>(in, a, stream);
-        return launch_persistent<32, 32, 3, false, 4, true, true>(in, a, stream);
+        if (c.persist == 7) return launch_persistent<32, 32, 2, false, 8, true, true>(in, a, stream, plan);
+        if (key == 64322) return launch_persistent<64, 32, 2, false, 4, true, true>(in, a, stream, plan);
+        return launch_persistent<32, 32, 3, false, 4, true, true>(in, a, stream, plan);
     }
     if (c.persist == 7)
         switch (key)
         {
-        case 32322: return launch_persistent<32, 32, 2, false, 8, true>(in, a, stream);
+        case 32322: return launch_persistent<32, 32, 2, false, 8, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 6)
         switch (key)
         {
-        case 64322: return launch_persistent<64, 32, 2, false, 4, true>(in, a, stream);
-        case 32323: return launch_persistent<32, 32, 3, false, 4, true>(in, a, stream);
+        case 64322: return launch_persistent<64, 32, 2, false, 4, true>(in, a, stream, plan);
+        case 32323: return launch_persistent<32, 32, 3, false, 4, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 5)
         switch (key)
         {
-        case 32164: return launch_persistent<32, 16, 4, true, 8, true>(in, a, stream);
-        case 32322: return launch_persistent<32, 32, 2, true, 8, true>(in, a, stream);
+        case 32164: return launch_persistent<32, 16, 4, true, 8, true>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2, true, 8, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 4)
         switch (key)
         {
-        case 32167: return launch_persistent<32, 16, 7, true, 4, true>(in, a, stream);
-        case 32323: return launch_persistent<32, 32, 3, true, 4, true>(in, a, stream);
-        case 64322: return launch_persistent<64, 32, 2, true, 4, true>(in, a, stream);
-        case 64323: return launch_persistent<64, 32, 3, true, 4, true>(in, a, stream);
+        case 32167: return launch_persistent<32, 16, 7, true, 4, true>(in, a, stream, plan);
+        case 32323: return launch_persistent<32, 32, 3, true, 4, true>(in, a, stream, plan);
+        case 64322: return launch_persistent<64, 32, 2, true, 4, true>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, true, 4, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 3)
         switch (key)
         {
-        case 32168: return launch_persistent<32, 16, 8, true, 4>(in, a, stream);
-        case 32323: return launch_persistent<32, 32, 3, true, 4>(in, a, stream);
-        case 32324: return launch_persistent<32, 32, 4, true, 4>(in, a, stream);
-        case 64323: return launch_persistent<64, 32, 3, true, 4>(in, a, stream);
+        case 32168: return launch_persistent<32, 16, 8, true, 4>(in, a, stream, plan);
+        case 32323: return launch_persistent<32, 32, 3, true, 4>(in, a, stream, plan);
+        case 32324: return launch_persistent<32, 32, 4, true, 4>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, true, 4>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 2)
         switch (key)
         {
-        case 32170: return launch_persistent<32, 16, 10, true>(in, a, stream);
-        case 32322: return launch_persistent<32, 32, 2, true>(in, a, stream);
-        case 32325: return launch_persistent<32, 32, 5, true>(in, a, stream);
-        case 32326: return launch_persistent<32, 32, 6, true>(in, a, stream);
-        case 64323: return launch_persistent<64, 32, 3, true>(in, a, stream);
-        case 64324: return launch_persistent<64, 32, 4, true>(in, a, stream);
+        case 32170: return launch_persistent<32, 16, 10, true>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2, true>(in, a, stream, plan);
+        case 32325: return launch_persistent<32, 32, 5, true>(in, a, stream, plan);
+        case 32326: return launch_persistent<32, 32, 6, true>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, true>(in, a, stream, plan);
+        case 64324: return launch_persistent<64, 32, 4, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist)
         switch (key)
         {
-        case 32164: return launch_persistent<32, 16, 4>(in, a, stream);
-        case 32322: return launch_persistent<32, 32, 2>(in, a, stream);
-        case 32324: return launch_persistent<32, 32, 4>(in, a, stream);
-        case 64164: return launch_persistent<64, 16, 4>(in, a, stream);
-        case 64322: return launch_persistent<64, 32, 2>(in, a, stream);
-        case 64323: return launch_persistent<64, 32, 3>(in, a, stream);
-        case 128163: return launch_persistent<128, 16, 3>(in, a, stream);
-        case 128322: return launch_persistent<128, 32, 2>(in, a, stream);
+        case 32164: return launch_persistent<32, 16, 4>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2>(in, a, stream, plan);
+        case 32324: return launch_persistent<32, 32, 4>(in, a, stream, plan);
+        case 64164: return launch_persistent<64, 16, 4>(in, a, stream, plan);
+        case 64322: return launch_persistent<64, 32, 2>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3>(in, a, stream, plan);
+        case 128163: return launch_persistent<128, 16, 3>(in, a, stream, plan);
+        case 128322: return launch_persistent<128, 32, 2>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     switch (key)
     {
-    case 32164: return launch<32, 16, 4>(in, a, stream);
-    case 32322: return launch<32, 32, 2>(in, a, stream);
-    case 32324: return launch<32, 32, 4>(in, a, stream);
-    case 64164: return launch<64, 16, 4>(in, a, stream);
-    case 64322: return launch<64, 32, 2>(in, a, stream);
-    case 64323: return launch<64, 32, 3>(in, a, stream);
-    case 128163: return launch<128, 16, 3>(in, a, stream);
-    case 128322: return launch<128, 32, 2>(in, a, stream);
+    case 32164: return launch<32, 16, 4>(in, a, stream, plan);
+    case 32322: return launch<32, 32, 2>(in, a, stream, plan);
+    case 32324: return launch<32, 32, 4>(in, a, stream, plan);
+    case 64164: return launch<64, 16, 4>(in, a, stream, plan);
+    case 64322: return launch<64, 32, 2>(in, a, stream, plan);
+    case 64323: return launch<64, 32, 3>(in, a, stream, plan);
+    case 128163: return launch<128, 16, 3>(in, a, stream, plan);
+    case 128322: return launch<128, 32, 2>(in, a, stream, plan);
     }
     return cudaErrorInvalidValue;
 }
 
 cudaError_t to_blocked_bf16(const float* x, int N, int C, int H, int W, __nv_bfloat16* out, int Cpad,
-                            cudaStream_t stream, bool log1p_in, bool skip_zero_blocks)
+                            cudaStream_t stream, bool log1p_in, bool skip_zero_blocks, int* clear)
 {
     const int nb = skip_zero_blocks ? (C + 7) / 8 : Cpad / 8;
     const size_t total = (size_t)N * nb * H * W;
     to_blocked_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(x, N, C, H, W, out, Cpad, nb,
-                                                                         log1p_in ? 1 : 0);
+                                                                         log1p_in ? 1 : 0, clear);
     return cudaGetLastError();
 }
 

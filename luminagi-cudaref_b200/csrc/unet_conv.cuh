@@ -117,8 +117,25 @@ ConvPackJob conv_pack_job_dgrad(const float* d_w, int Cout, int Cin_real, int ci
 // Packs up to kMaxPackJobs layers in one launch (forward jobs: the same bits as one conv_pack_weights call each).
 cudaError_t conv_pack_many(const ConvPackJob* jobs, int n, cudaStream_t stream);
 
-// Launches the convolution reading `in` (blocked BF16, N x Cin x H x W).
-cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream);
+// What a launch needs beside its arguments, kept per layer by a caller that runs the same layer again: the tensor
+// maps and the grid, which follow from the key alone (buffers, sizes, tile).
+struct ConvPlan
+{
+    struct Key
+    {
+        const void *in, *up_h;
+        int N, H, W, Cin, Cout, up_C;
+        ConvTile tile;
+    } key{};
+    bool ready = false;
+    CUtensorMap m, m2;
+    int a_chunked = 0, smem = 0;
+    unsigned grid[3] = {0, 0, 0};
+};
+
+// Launches the convolution reading `in` (blocked BF16, N x Cin x H x W).  plan (optional) is filled on the first
+// call and whenever its key differs.
+cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan* plan = nullptr);
 
 // The bounded wait of the convolution kernels (tc::mbar_wait) on an mbarrier
 // that nothing arrives at: after limit_ns the probe stores 3 in *err, as a
@@ -131,8 +148,10 @@ cudaError_t launch_wait_probe(int* err, unsigned long long limit_ns, cudaStream_
 // log1p_in applies log1p to every value first (the HDR variant's input).
 // skip_zero_blocks: leave the 8-channel blocks past channel C untouched (the
 // caller keeps them zero).
+// clear (optional): an int set to 0.
 cudaError_t to_blocked_bf16(const float* x, int N, int C, int H, int W, __nv_bfloat16* out, int Cpad,
-                            cudaStream_t stream, bool log1p_in = false, bool skip_zero_blocks = false);
+                            cudaStream_t stream, bool log1p_in = false, bool skip_zero_blocks = false,
+                            int* clear = nullptr);
 
 // Bilinear 2x upsampling (F.interpolate(scale_factor=2, mode="bilinear",
 // align_corners=False)) of a blocked BF16 tensor N x C x h x w into channels

@@ -84,11 +84,13 @@ struct lg_unet
     // tile shapes (lg::ConvTile; zero = the default heuristic) of the 14 convs and
     // the 16 input-gradient convs, as chosen by lg_unet_autotune
     lg::ConvTile tile[14] = {}, tile_dg[16] = {};
+    // launch plans of the convs (rebuilt when buffers, sizes or tiles change)
+    lg::ConvPlan plan[14], plan_dg[16];
     // autotuning: events recorded around one conv of the forward (probe_layer)
     // or of the backward (probe_dgrad); -1 = none
     int probe_layer = -1, probe_dgrad = -1;
     cudaEvent_t probe_ev0 = nullptr, probe_ev1 = nullptr;
-    cudaEvent_t order_ev = nullptr;  // lg_unet_train_step_async: orders the caller's stream and the network's
+    cudaEvent_t order_ev = nullptr;  // calls with a stream: orders the caller's stream and the network's
 };
 
 namespace lg

@@ -286,7 +286,7 @@ int loss_and_grads(lg_unet* u, const float* d_x, const float* d_t, int N, int H,
         a.tile = u->tile_dg[k];
         const bool probe = k == u->probe_dgrad;
         if (probe) LG_TRY_CUDA(cudaEventRecord(u->probe_ev0, st));
-        LG_TRY_CUDA(conv3x3_forward((const bf*)u->dz[d.layer].p, a, st));
+        LG_TRY_CUDA(conv3x3_forward((const bf*)u->dz[d.layer].p, a, st, &u->plan_dg[k]));
         if (probe) LG_TRY_CUDA(cudaEventRecord(u->probe_ev1, st));
         return LG_OK;
     };
