@@ -22,7 +22,7 @@ __device__ __forceinline__ uint64_t global_timer_ns()
 }
 
 // Programmatic dependent launch: let the next kernel of the stream start its
-// blocks as soon as this grid's have all started, and wait until the kernels
+// blocks once every block of this grid has called this or ended, and wait until the kernels
 // before this one have finished and their writes are visible (a no-op in a
 // launch without the attribute).
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -301,6 +301,10 @@ void lg_unet_destroy(lg_unet* u)
     if (u->probe_ev0) cudaEventDestroy(u->probe_ev0);
     if (u->probe_ev1) cudaEventDestroy(u->probe_ev1);
     if (u->order_ev) cudaEventDestroy(u->order_ev);
+    if (u->side) cudaStreamSynchronize(u->side);
+    if (u->side_ev) cudaEventDestroy(u->side_ev);
+    if (u->side_done) cudaEventDestroy(u->side_done);
+    if (u->side) cudaStreamDestroy(u->side);
     if (u->stream) cudaStreamDestroy(u->stream);
     delete u;
 }

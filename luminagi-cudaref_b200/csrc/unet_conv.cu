@@ -425,7 +425,6 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
     __shared__ EpiConsts ec;
 
     const int tid = threadIdx.x, warp = tid >> 5;
-    tc::launch_dependents();
     const int n_cot = a.Cout / BN;
     const int x0 = blockIdx.x * kTileX;
     const int y0 = blockIdx.y * kRows;
@@ -516,6 +515,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
             if (a.err) atomicExch(a.err, 1);
         }
         tc::mma_commit(done);  // completes when every MMA issued above has finished
+        tc::launch_dependents();
     }
     __syncwarp();
     // Epilogue: every thread owns TMEM lane = pixel x0 + tid.
@@ -621,7 +621,6 @@ __global__ void __launch_bounds__(kPThreads, 1) conv3x3_tc_persistent(const __gr
     __shared__ EpiConsts ec;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    tc::launch_dependents();
     const int n_cot = a.Cout / BN;
     const int tiles_x = (a.W + kTileX - 1) / kTileX, tiles_y = (a.H + ROWS - 1) / ROWS;
     const int n_tiles = tiles_x * tiles_y * a.N * n_cot;
@@ -865,6 +864,11 @@ __global__ void __launch_bounds__(kPThreads, 1) conv3x3_tc_persistent(const __gr
                 tc::mma_commit(&acc_full[b]);
             }
             tc::mma_commit(done);  // completes when every MMA issued above has finished
+            // only the last tiles' epilogues are left: the next layer's blocks may take their places.  (From the
+            // start of the kernel on, they would sit on SMs that other streams' kernels could use: three networks
+            // side by side at 1x256x512 then took 121 us
+            // a pass instead of 111, and one alone 236 instead of 226.)
+            tc::launch_dependents();
         }
     }
     else

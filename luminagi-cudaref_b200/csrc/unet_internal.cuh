@@ -84,6 +84,9 @@ struct lg_unet
     // tile shapes (lg::ConvTile; zero = the default heuristic) of the 14 convs and
     // the 16 input-gradient convs, as chosen by lg_unet_autotune
     lg::ConvTile tile[14] = {}, tile_dg[16] = {};
+    // second stream of the backward pass (weight, bias and tail gradients) and the events that order the two
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_ev = nullptr, side_done = nullptr;
     // launch plans of the convs (rebuilt when buffers, sizes or tiles change)
     lg::ConvPlan plan[14], plan_dg[16];
     // autotuning: events recorded around one conv of the forward (probe_layer)

@@ -222,6 +222,39 @@ int loss_and_grads(lg_unet* u, const float* d_x, const float* d_t, int N, int H,
     LG_TRY(unet_forward_device(u, d_x, N, H, W, (float*)u->yout.p));
     LG_TRY(pack_dgrad(u));
     cudaStream_t st = u->stream;
+    // Weight, bias and tail gradients are read by nothing in the pass: they run on a second stream beside the
+    // chain of input gradients, each once the gradient it reads is there.
+    if (!u->side)
+    {
+        LG_TRY_CUDA(cudaStreamCreateWithFlags(&u->side, cudaStreamNonBlocking));
+        LG_TRY_CUDA(cudaEventCreateWithFlags(&u->side_ev, cudaEventDisableTiming));
+        LG_TRY_CUDA(cudaEventCreateWithFlags(&u->side_done, cudaEventDisableTiming));
+    }
+    // (the autotuner times one input gradient at a time: nothing runs beside it then)
+    cudaStream_t side = u->probe_dgrad >= 0 ? st : u->side;
+    // st waits for the side stream before this function returns, errors included, so later work on st (the next
+    // pass overwrites what the side stream reads) is ordered after both.
+    struct Join
+    {
+        lg_unet* u;
+        cudaStream_t st, side;
+        bool joined;
+        cudaError_t join()
+        {
+            joined = true;
+            const cudaError_t e = cudaEventRecord(u->side_done, side);
+            return e == cudaSuccess ? cudaStreamWaitEvent(st, u->side_done, 0) : e;
+        }
+        ~Join()
+        {
+            if (!joined && join() != cudaSuccess) cudaStreamSynchronize(side);
+        }
+    } both{u, st, side, false};
+    auto follow = [&]() -> int {  // the side stream waits for everything on st so far
+        LG_TRY_CUDA(cudaEventRecord(u->side_ev, st));
+        LG_TRY_CUDA(cudaStreamWaitEvent(side, u->side_ev, 0));
+        return LG_OK;
+    };
     float* G = (float*)u->grads.p;
     const float* P = (const float*)u->params.p;
     LG_TRY_CUDA(cudaMemsetAsync(G, 0, u->n_params * sizeof(float), st));
@@ -234,7 +267,8 @@ int loss_and_grads(lg_unet* u, const float* d_x, const float* d_t, int N, int H,
         (const bf*)u->u1.p, d_x, u->in_ch, u->log_hdr ? 1 : 0, d_t, P + u->tail_w_off, P + u->tail_b_off, N, H, W, u->slope, inv_numel,
         (bf*)u->dz[13].p, (float*)u->tpart.p);
     LG_TRY_CUDA(cudaGetLastError());
-    tail_reduce_kernel<<<1, 128, 0, st>>>((const float*)u->tpart.p, tail_blocks, G + u->tail_w_off,
+    LG_TRY(follow());
+    tail_reduce_kernel<<<1, 128, 0, side>>>((const float*)u->tpart.p, tail_blocks, G + u->tail_w_off,
                                           G + u->tail_b_off, (float*)u->loss.p);
     LG_TRY_CUDA(cudaGetLastError());
 
@@ -243,7 +277,9 @@ int loss_and_grads(lg_unet* u, const float* d_x, const float* d_t, int N, int H,
     // forward inputs of each layer (blocked BF16)
     const void* in_of[14] = {u->x0.p, u->t1.p, u->p1.p, u->t2.p, u->p2.p, u->t3.p, u->p3.p,
                              u->t4.p, u->cat3.p, u->t5.p, u->cat2.p, u->t6.p, u->cat1.p, u->t7.p};
+    // queued right after the kernel that writes the layer's dZ
     auto wgrad = [&](int L) -> int {
+        LG_TRY(follow());
         const int lv = lv_out[L];
         WgradArgs a{};
         a.N = N;
@@ -257,7 +293,7 @@ int loss_and_grads(lg_unet* u, const float* d_x, const float* d_t, int N, int H,
         LG_TRY(u->wpart.ensure(conv3x3_wgrad_partial_floats(N, a.H, a.Cout, a.Cin, a.Cin_real, u->sm_count) *
                                sizeof(float)));
         a.partial = (float*)u->wpart.p;
-        LG_TRY_CUDA(conv3x3_wgrad((const bf*)u->dz[L].p, (const bf*)in_of[L], a, u->sm_count, st));
+        LG_TRY_CUDA(conv3x3_wgrad((const bf*)u->dz[L].p, (const bf*)in_of[L], a, u->sm_count, side));
         return LG_OK;
     };
     auto dgrad = [&](int k, void* out, int out_c, const void* ref, int ref_c, int ref_coff, const void* skip,
@@ -306,19 +342,19 @@ int loss_and_grads(lg_unet* u, const float* d_x, const float* d_t, int N, int H,
         return LG_OK;
     };
     LG_TRY(up_grad(1, 11, u->cat1.p, 96, u->lo11, 64, H / 2, W / 2));
-    LG_TRY(dgrad(2, u->gs1.p, 32, nullptr, 0, 0, nullptr, 0));
     LG_TRY(wgrad(11));
+    LG_TRY(dgrad(2, u->gs1.p, 32, nullptr, 0, 0, nullptr, 0));
     LG_TRY(dgrad(3, u->dz[10].p, 64, u->t6.p, 64, 0, nullptr, 0));
     LG_TRY(wgrad(10));
     LG_TRY(up_grad(4, 9, u->cat2.p, 192, u->lo9, 128, H / 4, W / 4));
-    LG_TRY(dgrad(5, u->gs2.p, 64, nullptr, 0, 0, nullptr, 0));
     LG_TRY(wgrad(9));
+    LG_TRY(dgrad(5, u->gs2.p, 64, nullptr, 0, 0, nullptr, 0));
     LG_TRY(dgrad(6, u->dz[8].p, 128, u->t5.p, 128, 0, nullptr, 0));
     LG_TRY(wgrad(8));
     LG_TRY(up_grad(7, 7, u->cat3.p, 384, u->lo7, 256, H / 8, W / 8));
+    LG_TRY(wgrad(7));
     LG_TRY(dgrad(8, u->gs3.p, 128, nullptr, 0, 0, nullptr, 0));
     // encoder
-    LG_TRY(wgrad(7));
     LG_TRY(dgrad(9, u->dz[6].p, 256, u->t4.p, 256, 0, nullptr, 0));
     LG_TRY(wgrad(6));
     LG_TRY(dgrad(10, u->dz[5].p, 128, u->cat3.p, 384, 256, u->gs3.p, 128));
@@ -343,7 +379,8 @@ int loss_and_grads(lg_unet* u, const float* d_x, const float* d_t, int N, int H,
         bias_c += kLayers[L].cout;
     }
     LG_TRY(u->bpart.ensure(conv_bias_grad_partial_floats(bias_c) * sizeof(float)));
-    LG_TRY_CUDA(conv_bias_grad_many(bj, 14, (float*)u->bpart.p, st));
+    LG_TRY_CUDA(conv_bias_grad_many(bj, 14, (float*)u->bpart.p, side));
+    LG_TRY_CUDA(both.join());
     if (loss_host)
     {
         float s = 0.0f;
