@@ -378,6 +378,19 @@ __device__ __forceinline__ void start_sample(PathState& st, const DevCam& cam)
     st.ray = primary_ray(cam, st.px, st.py, jx, jy);
 }
 
+// A point light's contribution is exactly zero from one radius on (its
+// attenuation is max(0, 1 - dist / radius) squared), while the reference casts
+// shadow rays up to three radii.  Whatever such a ray would find, it adds
+// throughput * 0 to the sum, so no ray is cast: same bits, as long as the
+// throughput is finite.  (The sun's ray is cast at any intensity, as in the
+// reference.)  On the engine frame (8 spp, 2 bounces; radii 15 and 12 m in a
+// 40 m scene) 65.4 -> 52.2 M rays and 34.5 -> 28.1 ms.
+__device__ __forceinline__ bool adds_nothing(const PathState& st)
+{
+    const float t = st.throughput.x + st.throughput.y + st.throughput.z;
+    return st.contrib.x == 0.0f && st.contrib.y == 0.0f && st.contrib.z == 0.0f && fabsf(t) < __int_as_float(0x7f800000);
+}
+
 // Consumes the result of the ray in flight and sets up the next one.
 // Returns false when the chunk's last sample has finished.  kAcc64: every
 // radiance term is also multiplied and added in FP64.
@@ -417,7 +430,8 @@ __device__ __forceinline__ bool advance(PathState& st, const DevScene& s, const 
     if (!path_done)
     {
         for (int next = st.li + 1; next <= s.n_points; ++next)
-            if (light_query(s, next, st.P, st.N, st.albedo, st.ray, st.tmax, st.contrib))
+            if (light_query(s, next, st.P, st.N, st.albedo, st.ray, st.tmax, st.contrib) &&
+                !(next > 0 && adds_nothing(st)))
             {
                 st.li = next;
                 return true;
