@@ -121,6 +121,7 @@ struct lg_renderer
     int tree_mode = LG_RENDER_TREE_PLOC_TRIANGLES;  // tree the traversal records are built from
     int tree_used = -1;                   // the mode actually built (PLOC falls back to the BuildBVH tree)
     DevBuf rnodes, rt_scratch;            // render tree (depth order) and its build scratch
+    DevBuf level_start;                   // first render-tree node of each depth
     bool watertight = false;  // ray/triangle test: Moller-Trumbore (the reference's) or watertight
     int trace_blocks_per_sm = 0;  // persistent trace grid (0 = occupancy maximum); see lg_renderer_autotune
     int trace_refill = LG_REFILL_DEFAULT;  // finished rays per warp that trigger the path logic (1..32)
@@ -254,7 +255,7 @@ int upload_common(lg_renderer* r, const lg_scene_desc* d)
 // Scratch of build_wide_nodes and build_wide4_nodes for a render tree of n nodes.
 size_t record_scratch_bytes(int n)
 {
-    return ((size_t)n * 11 + 2 * ((size_t)n / 1024 + 1) + 256) * sizeof(int);
+    return ((size_t)n * 9 + 2 * ((size_t)n / 1024 + 1) + 256) * sizeof(int);
 }
 
 // Traversal records (2- and 4-wide) from the render tree tree_mode selects
@@ -269,33 +270,39 @@ int build_records(lg_renderer* r)
     LG_TRY(r->rnodes.reserve(cap * sizeof(lg_bvh_node)));
     LG_TRY(r->rt_scratch.reserve(render_tree_scratch_bytes(nbvh, r->n_tris)));
     int mode = r->tree_mode;
+    LG_TRY(r->level_start.reserve(257 * sizeof(int)));
+    int levels = 1, level_start[257];
     int rc = build_render_tree(r->nodes.as<lg_bvh_node>(), nbvh, r->tris.as<lg_triangle>(), r->n_tris, mode,
-                               r->rnodes.as<lg_bvh_node>(), r->rt_scratch.p, r->rt_scratch.bytes, r->stream);
+                               r->rnodes.as<lg_bvh_node>(), r->level_start.as<int>(), level_start, &levels, r->rt_scratch.p,
+                               r->rt_scratch.bytes, r->stream);
     if (rc != LG_OK && mode != LG_RENDER_TREE_BUILDBVH)
     {
         // e.g. leaves whose triangle ranges share a first triangle: keep the given topology
         mode = LG_RENDER_TREE_BUILDBVH;
         rc = build_render_tree(r->nodes.as<lg_bvh_node>(), nbvh, r->tris.as<lg_triangle>(), r->n_tris, mode,
-                               r->rnodes.as<lg_bvh_node>(), r->rt_scratch.p, r->rt_scratch.bytes, r->stream);
+                               r->rnodes.as<lg_bvh_node>(), r->level_start.as<int>(), level_start, &levels, r->rt_scratch.p,
+                               r->rt_scratch.bytes, r->stream);
     }
     LG_TRY(rc);
     r->tree_used = mode;
     const int n = render_tree_nodes(nbvh, r->n_tris, mode);
     LG_TRY(r->scratch.reserve(record_scratch_bytes(n)));
     LG_TRY(r->wide4.reserve(((size_t)n / 2 + 1) * sizeof(Wide4Node)));
-    int root = 0, ni = 0, nl = 0, root4 = 0, n4 = 0;
+    int root = 0, n4 = 0;
+    const int nl = (n + 1) / 2;  // n = 2 * leaves - 1
     LG_TRY_CUDA(build_wide_nodes(r->rnodes.as<lg_bvh_node>(), n, r->wide.as<WideNode>(), r->leaves.as<int2>(),
-                                 r->scratch.as<int>(), &root, &ni, &nl, r->stream));
+                                 r->scratch.as<int>(), r->stream));
     int leaf_inline = 0;
     static const int2 kEmptyLeaf = {0, 0};
     LG_TRY_CUDA(cudaMemcpyAsync(r->leaves.as<int2>() + nl, &kEmptyLeaf, sizeof(int2), cudaMemcpyHostToDevice,
                                 r->stream));
-    LG_TRY_CUDA(build_wide4_nodes(r->rnodes.as<lg_bvh_node>(), n, r->n_tris, nl, r->wide4.as<Wide4Node>(),
-                                  r->scratch.as<int>(), &root4, &n4, &leaf_inline, &r->stack4, &r->stack2, r->stream));
+    LG_TRY_CUDA(build_wide4_nodes(r->rnodes.as<lg_bvh_node>(), n, r->n_tris, nl, level_start, levels,
+                                  r->wide4.as<Wide4Node>(), r->scratch.as<int>(), &root, &n4, &leaf_inline, &r->stack4,
+                                  &r->stack2, r->stream));
     LG_TRY_CUDA(cudaStreamSynchronize(r->stream));
     r->leaf_inline = leaf_inline;
-    r->root4 = root4;
-    r->n4 = root4 >= 0 ? n4 : 0;
+    r->root4 = root;
+    r->n4 = root >= 0 ? n4 : 0;
     r->root = root;
     ++r->scene_gen;
     return r->l2_window ? apply_l2_window(r) : LG_OK;
@@ -765,7 +772,7 @@ void lg_renderer_destroy(lg_renderer* r)
     if (r->fault_host) cudaFreeHost(r->fault_host);
     r->fault.release();
     r->matchk.release();
-    for (DevBuf* b : {&r->batch_jobs, &r->batch_acc, &r->batch_rgb, &r->rnodes, &r->rt_scratch, &r->wf_scratch})
+    for (DevBuf* b : {&r->batch_jobs, &r->batch_acc, &r->batch_rgb, &r->rnodes, &r->rt_scratch, &r->level_start, &r->wf_scratch})
         b->release();
     for (DevBuf* b : {&r->tris, &r->tris_in, &r->nodes, &r->wide, &r->wide4, &r->leaves, &r->tv, &r->mats, &r->points,
                       &r->scratch, &r->accum, &r->accum64, &r->rgb, &r->work, &r->counters})

@@ -135,18 +135,37 @@ __global__ void rank_kernel(const uint32_t* __restrict__ order, int n, int* __re
     const int r = blockIdx.x * kTB + threadIdx.x;
     if (r < n) newpos[order[r]] = r;
 }
-__global__ void emit_kernel(const lg_bvh_node* __restrict__ in, const uint32_t* __restrict__ order,
-                            const int* __restrict__ newpos, int n, lg_bvh_node* __restrict__ out)
+// Nodes in depth order with their links renumbered, word by word (a node is 10
+// words): whole sectors written.  One thread per node took 91 us for 2.1 M
+// nodes, this 51.
+constexpr int kEmitNodes = 256;
+__global__ void __launch_bounds__(kTB) emit_kernel(const lg_bvh_node* __restrict__ in, const uint32_t* __restrict__ order,
+                                                   const int* __restrict__ newpos, int n, lg_bvh_node* __restrict__ out)
 {
-    const int r = blockIdx.x * kTB + threadIdx.x;
-    if (r >= n) return;
-    lg_bvh_node nd = in[order[r]];
-    if (nd.triCount == 0)
+    __shared__ uint32_t s_src[kEmitNodes];
+    const int base = blockIdx.x * kEmitNodes, cnt = min(kEmitNodes, n - base);
+    for (int i = threadIdx.x; i < cnt; i += kTB) s_src[i] = order[base + i];
+    __syncthreads();
+    const int* words = reinterpret_cast<const int*>(in);
+    int* to = reinterpret_cast<int*>(out) + (size_t)base * 10;
+#pragma unroll 5
+    for (int w = threadIdx.x; w < cnt * 10; w += kTB)
     {
-        nd.left = newpos[nd.left];
-        nd.right = newpos[nd.right];
+        const int i = w / 10, o = w - 10 * i;
+        const size_t at = (size_t)s_src[i] * 10;
+        int v = words[at + o];
+        if ((o == 6 || o == 7) && words[at + 9] == 0) v = newpos[v];  // left, right of an internal node
+        to[w] = v;
     }
-    out[r] = nd;
+}
+// Where each depth's nodes begin in depth order, from the sort's counts of the 256 depths; start[256] = n.
+__global__ void level_start_kernel(const uint32_t* __restrict__ counts, int n, int* __restrict__ start)
+{
+    __shared__ int ws[kTB / 32];
+    int total;
+    const int e = block_excl_scan((int)counts[threadIdx.x], ws, total);
+    start[threadIdx.x] = e;
+    if (threadIdx.x == 0) start[256] = n;
 }
 
 // ---- PLOC ----
@@ -291,38 +310,61 @@ __global__ void round_flags_kernel(const int* __restrict__ nn, const int* __rest
         ksums[blockIdx.x] = tk;
     }
 }
-__global__ void round_sums_kernel(int* __restrict__ msums, int* __restrict__ ksums, int nb, const int* __restrict__ cur,
-                                  int* __restrict__ nxt)
+constexpr int kSumThreads = 1024;
+__global__ void __launch_bounds__(kSumThreads) round_sums_kernel(int* __restrict__ msums, int* __restrict__ ksums, int nb,
+                                                                 const int* __restrict__ cur, int* __restrict__ nxt)
 {
-    __shared__ int ws[kTB / 32];
-    __shared__ int carry[2];
-    if (threadIdx.x < 2) carry[threadIdx.x] = 0;
-    __syncthreads();
-    for (int b = 0; b < nb; b += kTB)
+    __shared__ int ws[2][kSumThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = (nb + kSumThreads - 1) / kSumThreads;  // consecutive entries per thread
+    const int first = min((int)threadIdx.x * per, nb), last = min(first + per, nb);
+    int sm = 0, sk = 0;
+    for (int i = first; i < last; ++i)
     {
-        const int i = b + threadIdx.x;
-        int tm, tk;
-        const int em = block_excl_scan(i < nb ? msums[i] : 0, ws, tm);
-        const int ek = block_excl_scan(i < nb ? ksums[i] : 0, ws, tk);
-        if (i < nb)
+        sm += msums[i];
+        sk += ksums[i];
+    }
+    int xm = sm, xk = sk;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int ym = __shfl_up_sync(0xffffffffu, xm, o), yk = __shfl_up_sync(0xffffffffu, xk, o);
+        if (lane >= o)
         {
-            msums[i] = carry[0] + em;
-            ksums[i] = carry[1] + ek;
+            xm += ym;
+            xk += yk;
         }
-        __syncthreads();
-        if (threadIdx.x == 0)
+    }
+    if (lane == 31)
+    {
+        ws[0][warp] = xm;
+        ws[1][warp] = xk;
+    }
+    __syncthreads();
+    int bm = xm - sm, bk = xk - sk, merges = 0, kept = 0;
+    for (int w = 0; w < kSumThreads / 32; ++w)
+    {
+        if (w == warp)
         {
-            carry[0] += tm;
-            carry[1] += tk;
+            bm += merges;
+            bk += kept;
         }
-        __syncthreads();
+        merges += ws[0][w];
+        kept += ws[1][w];
+    }
+    for (int i = first; i < last; ++i)
+    {
+        const int m = msums[i], k = ksums[i];
+        msums[i] = bm;
+        ksums[i] = bk;
+        bm += m;
+        bk += k;
     }
     if (threadIdx.x == 0)
     {
-        const int merges = carry[0];
         nxt[2] = cur[2] | ((cur[0] > 1 && merges == 0) ? 1 : 0);
         nxt[1] = cur[1] + merges;
-        nxt[0] = carry[1];
+        nxt[0] = kept;
     }
 }
 __global__ void round_apply_kernel(const int* __restrict__ nn, const int* __restrict__ cur,
@@ -358,6 +400,165 @@ __global__ void round_apply_kernel(const int* __restrict__ nn, const int* __rest
         const int pos = ksums[blockIdx.x] + kpos[i];
         cid2[pos] = id;
         cbox2[pos] = b;
+    }
+}
+
+// Every remaining round at once, in one block, from kTailClusters clusters on:
+// the rounds above in shared memory, with the same neighbours, merges and
+// numbering.  On the engine scene 40 of the 64 rounds start with fewer clusters
+// than that: 189 us here, about 600 us as four launches of 3 to 4 us each.
+constexpr int kTailClusters = 4096;
+constexpr int kTailThreads = 1024;
+constexpr int kTailItems = kTailClusters / kTailThreads;
+struct TailShared
+{
+    float box[6][kTailClusters];
+    int nn[kTailClusters], id[kTailClusters];
+    int merges[kTailItems * kTailThreads / 32], keeps[kTailItems * kTailThreads / 32];  // per 32 clusters
+    int total[2];
+};
+__global__ void __launch_bounds__(kTailThreads) rounds_tail_kernel(const int* __restrict__ cid, const Box* __restrict__ cbox,
+                                                                   int* __restrict__ state, lg_bvh_node* __restrict__ tn,
+                                                                   int* __restrict__ root)
+{
+    extern __shared__ __align__(16) unsigned char tail_mem[];
+    TailShared& sh = *reinterpret_cast<TailShared*>(tail_mem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    int c = state[0], next_id = state[1];
+    if (c > kTailClusters) return;  // the host never launches it so
+    auto box_at = [&](int i) {
+        Box b;
+        b.lo = make_float4(sh.box[0][i], sh.box[1][i], sh.box[2][i], 0.0f);
+        b.hi = make_float4(sh.box[3][i], sh.box[4][i], sh.box[5][i], 0.0f);
+        return b;
+    };
+    auto put_box = [&](int i, const Box& b) {
+        sh.box[0][i] = b.lo.x;
+        sh.box[1][i] = b.lo.y;
+        sh.box[2][i] = b.lo.z;
+        sh.box[3][i] = b.hi.x;
+        sh.box[4][i] = b.hi.y;
+        sh.box[5][i] = b.hi.z;
+    };
+    for (int i = tid; i < c; i += kTailThreads)
+    {
+        put_box(i, cbox[i]);
+        sh.id[i] = cid[i];
+    }
+    __syncthreads();
+    while (c > 1)
+    {
+        for (int i = tid; i < c; i += kTailThreads)
+        {
+            const Box bi = box_at(i);
+            float best = __int_as_float(0x7f800000);
+            int bj = -1;
+            const int lo = max(0, i - kRadius), hi = min(c - 1, i + kRadius);
+            for (int j = lo; j <= hi; ++j)
+            {
+                if (j == i) continue;
+                const float a = half_area(join(bi, box_at(j)));
+                if (a < best)
+                {
+                    best = a;
+                    bj = j;
+                }
+            }
+            sh.nn[i] = bj;
+        }
+        __syncthreads();
+        Box b[kTailItems];
+        int id[kTailItems], rank_m[kTailItems], rank_k[kTailItems], partner[kTailItems];
+        bool keep[kTailItems];
+#pragma unroll
+        for (int k = 0; k < kTailItems; ++k)
+        {
+            const int i = k * kTailThreads + tid;
+            bool m = false;
+            keep[k] = false;
+            partner[k] = -1;
+            if (i < c)
+            {
+                const int j = sh.nn[i];
+                const bool mutual = j >= 0 && sh.nn[j] == i;
+                m = mutual && i < j;
+                keep[k] = !(mutual && i > j);
+                if (m) partner[k] = j;
+                b[k] = box_at(i);
+                id[k] = sh.id[i];
+            }
+            const unsigned vm = __ballot_sync(0xffffffffu, m), vk = __ballot_sync(0xffffffffu, keep[k]);
+            rank_m[k] = __popc(vm & lt);
+            rank_k[k] = __popc(vk & lt);
+            if (lane == 0)
+            {
+                sh.merges[k * (kTailThreads / 32) + warp] = __popc(vm);
+                sh.keeps[k * (kTailThreads / 32) + warp] = __popc(vk);
+            }
+        }
+        __syncthreads();
+        // exclusive scans of the counts of 32: warp 0 the merges, warp 1 the kept clusters
+        if (warp < 2)
+        {
+            int* v = warp == 0 ? sh.merges : sh.keeps;
+            int carry = 0;
+            for (int at = lane; at < kTailItems * kTailThreads / 32; at += 32)
+            {
+                const int own = v[at];
+                int x = own;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1)
+                {
+                    const int y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                v[at] = carry + x - own;
+                carry += __shfl_sync(0xffffffffu, x, 31);
+            }
+            if (lane == 0) sh.total[warp] = carry;
+        }
+        __syncthreads();
+        const int merges = sh.total[0], kept = sh.total[1];
+        if (merges == 0)
+        {
+            if (tid == 0) state[2] = 1;
+            return;
+        }
+#pragma unroll
+        for (int k = 0; k < kTailItems; ++k)
+        {
+            if (partner[k] < 0) continue;
+            const int j = partner[k];
+            b[k] = join(b[k], box_at(j));
+            lg_bvh_node nd;
+            nd.bbMin[0] = b[k].lo.x; nd.bbMin[1] = b[k].lo.y; nd.bbMin[2] = b[k].lo.z;
+            nd.bbMax[0] = b[k].hi.x; nd.bbMax[1] = b[k].hi.y; nd.bbMax[2] = b[k].hi.z;
+            nd.left = id[k];
+            nd.right = sh.id[j];
+            nd.firstTri = -1;
+            nd.triCount = 0;
+            id[k] = next_id + sh.merges[k * (kTailThreads / 32) + warp] + rank_m[k];
+            tn[id[k]] = nd;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kTailItems; ++k)
+            if (keep[k])
+            {
+                const int pos = sh.keeps[k * (kTailThreads / 32) + warp] + rank_k[k];
+                put_box(pos, b[k]);
+                sh.id[pos] = id[k];
+            }
+        next_id += merges;
+        c = kept;
+        __syncthreads();
+    }
+    if (tid == 0)
+    {
+        state[0] = c;
+        state[1] = next_id;
+        *root = sh.id[0];
     }
 }
 
@@ -398,7 +599,8 @@ size_t render_tree_scratch_bytes(int n_nodes, int n_tris)
 }
 
 int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle* d_tris, int n_tris, int mode,
-                      lg_bvh_node* d_out, void* scratch, size_t scratch_bytes, cudaStream_t st)
+                      lg_bvh_node* d_out, int* d_level_start, int* level_start_host, int* levels, void* scratch,
+                      size_t scratch_bytes, cudaStream_t st)
 {
     if (n_nodes <= 0) return LG_OK;
     const int in_nodes = n_nodes;
@@ -461,7 +663,7 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
         int cur = 0;
         int hstate[3] = {c, L, 0};
         LG_TRY_CUDA(cudaMemcpyAsync(sbuf[0], hstate, sizeof(hstate), cudaMemcpyHostToDevice, st));
-        while (hstate[0] > 1)
+        while (hstate[0] > kTailClusters)
         {
             const int gc = (hstate[0] + kTB - 1) / kTB;
             for (int k = 0; k < kRoundsPerCheck; ++k)
@@ -470,7 +672,7 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
                 int* sn = sbuf[cur ^ 1];
                 nn_kernel<<<gc, kTB, 0, st>>>(cbox, sc, nn);
                 round_flags_kernel<<<gc, kTB, 0, st>>>(nn, sc, mflag, kflag, midx, kpos, sums, ksums);
-                round_sums_kernel<<<1, kTB, 0, st>>>(sums, ksums, gc, sc, sn);
+                round_sums_kernel<<<1, kSumThreads, 0, st>>>(sums, ksums, gc, sc, sn);
                 round_apply_kernel<<<gc, kTB, 0, st>>>(nn, sc, mflag, kflag, midx, kpos, sums, ksums, cid, cbox, tn,
                                                        cid2, cbox2);
                 LG_TRY_CUDA(cudaGetLastError());
@@ -482,10 +684,17 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
             LG_TRY_CUDA(cudaStreamSynchronize(st));
             if (hstate[2]) return set_error(LG_ERR_DEVICE, "render tree: a clustering round merged nothing");
         }
+        int* droot = totals + 24;
+        LG_TRY_CUDA(cudaFuncSetAttribute((const void*)rounds_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(TailShared)));
+        rounds_tail_kernel<<<1, kTailThreads, sizeof(TailShared), st>>>(cid, cbox, sbuf[cur], tn, droot);
+        LG_TRY_CUDA(cudaGetLastError());
+        LG_TRY_CUDA(cudaMemcpyAsync(hstate, sbuf[cur], sizeof(hstate), cudaMemcpyDeviceToHost, st));
+        LG_TRY_CUDA(cudaMemcpyAsync(&root, droot, sizeof(int), cudaMemcpyDeviceToHost, st));
+        LG_TRY_CUDA(cudaStreamSynchronize(st));
+        if (hstate[2]) return set_error(LG_ERR_DEVICE, "render tree: a clustering round merged nothing");
         const int next_id = hstate[1];
         if (next_id != n_nodes) return set_error(LG_ERR_DEVICE, "render tree: %d nodes, %d expected", next_id, n_nodes);
-        LG_TRY_CUDA(cudaMemcpyAsync(&root, cid, sizeof(int), cudaMemcpyDeviceToHost, st));
-        LG_TRY_CUDA(cudaStreamSynchronize(st));
         src = tn;
     }
     // Depth order: a stable sort of node ids by depth (ids ascending within a depth).
@@ -499,11 +708,14 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
     LG_TRY_CUDA(cudaMemcpyAsync(&sort_error, rs.error, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     LG_TRY_CUDA(cudaMemcpyAsync(&max_depth, depth + n_nodes - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     rank_kernel<<<g, kTB, 0, st>>>(ids, n_nodes, newpos);
-    emit_kernel<<<g, kTB, 0, st>>>(src, ids, newpos, n_nodes, d_out);
+    emit_kernel<<<(n_nodes + kEmitNodes - 1) / kEmitNodes, kTB, 0, st>>>(src, ids, newpos, n_nodes, d_out);
+    level_start_kernel<<<1, kTB, 0, st>>>(rs.hist, n_nodes, d_level_start);
+    LG_TRY_CUDA(cudaMemcpyAsync(level_start_host, d_level_start, 257 * sizeof(int), cudaMemcpyDeviceToHost, st));
     LG_TRY_CUDA(cudaGetLastError());
     LG_TRY_CUDA(cudaStreamSynchronize(st));
     if (sort_error) return set_error(LG_ERR_DEVICE, "render tree: a wait of the sort ran out");
     if (max_depth >= 255u) return set_error(LG_ERR_CAPACITY, "render tree: depth over 254");
+    *levels = (int)max_depth + 1;
     return LG_OK;
 }
 }  // namespace lg

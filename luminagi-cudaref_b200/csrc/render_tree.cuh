@@ -15,7 +15,9 @@ int render_tree_nodes(int n_nodes, int n_tris, int mode);
 // mode 0: d_nodes re-sorted by depth; mode 1: d_nodes' leaves regrouped by
 // PLOC; mode 2: PLOC over the triangles (d_tris, BVH order), one per leaf;
 // all sorted by depth.  d_out holds render_tree_nodes(...) records, root
-// first.  Returns an LG_* status (the message in lg_last_error).
+// first.  d_level_start (257 ints, device) and its host copy: the first node
+// of each depth, and n past the last; *levels: the number of depths.  Returns an LG_* status (the
+// message in lg_last_error).
 int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle* d_tris, int n_tris, int mode,
-                      lg_bvh_node* d_out, void* scratch, size_t scratch_bytes, cudaStream_t stream);
+                      lg_bvh_node* d_out, int* d_level_start, int* level_start_host, int* levels, void* scratch, size_t scratch_bytes, cudaStream_t stream);
 }  // namespace lg

@@ -124,27 +124,29 @@ struct TraceJob
 // Camera set-up of RenderSceneCUDA (pathtracer.cu:654-663); tanf runs on the host as there.
 DevCam make_dev_cam(const lg_camera& c);
 
-// Converts the reference node array (BFS) to WideNode records + leaf table.
-// Scratch: 2 * n_nodes ints.  Returns the root link through *root (device
-// write of one int; caller copies back) -- done inside the launcher.
+// Converts a node array in depth order (2L - 1 nodes for L leaves) to WideNode
+// records + leaf table.  Scratch: 2 * n_nodes ints and the scan's block sums.
 cudaError_t build_wide_nodes(const lg_bvh_node* d_nodes, int n_nodes, WideNode* d_wide, int2* d_leaves,
-                             int* d_scratch, int* root_host, int* n_internal_host, int* n_leaves_host,
-                             cudaStream_t stream);
-// Collapses the binary BVH (BFS order) into 4-wide records, top-down: a
-// record starts from its node's two children and repeatedly opens the
+                             int* d_scratch, cudaStream_t stream);
+// Collapses the binary BVH (depth order; level_start, on the host: the first
+// node of each of its `levels` depths, and the end) into 4-wide records,
+// top-down: a record starts from its node's two children and repeatedly opens the
 // internal child of largest surface area until it has four; the internal
 // children are the next records.  Records are numbered by the BFS rank of
 // their nodes (deterministic).  Must follow build_wide_nodes on the same
-// scratch (it reuses the leaf numbering).  Scratch: 11 * n_nodes + 256 ints.
+// scratch (it reuses the leaf numbering).  Scratch: 9 * n_nodes ints and the scans' block
+// sums.
+// root_host: the root link of both record forms (0 = record 0, ~0 = leaf 0).
 // null_leaf: the index of a leaf-table entry (0, 0) for absent children.
 // stack4_host / stack2_host: the most traversal-stack entries any ray can
 // need over the 4-wide records (the largest sum, over a root-to-record path,
 // of each record's child count less one: a visit stacks at most the hit
 // children it does not enter, and entries above a popped one are gone) and
 // over the 2-wide ones (the deepest internal node's depth + 1).
-cudaError_t build_wide4_nodes(const lg_bvh_node* d_nodes, int n_nodes, int n_tris, int null_leaf, Wide4Node* d_wide4,
-                              int* d_scratch, int* root4_host, int* n4_host, int* leaf_inline_host,
-                              int* stack4_host, int* stack2_host, cudaStream_t stream);
+cudaError_t build_wide4_nodes(const lg_bvh_node* d_nodes, int n_nodes, int n_tris, int null_leaf,
+                              const int* level_start, int levels, Wide4Node* d_wide4, int* d_scratch, int* root_host,
+                              int* n4_host, int* leaf_inline_host, int* stack4_host, int* stack2_host,
+                              cudaStream_t stream);
 // Intersection records, 3 float4 per triangle (w of the first = material):
 // (v0, v1-v0, v2-v0) for Moller-Trumbore, (v0, v1, v2) for the watertight test.
 cudaError_t prepare_triangles(const lg_triangle* d_tris, int n, float4* d_tv, bool watertight, cudaStream_t stream);
