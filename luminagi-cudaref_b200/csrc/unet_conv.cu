@@ -251,14 +251,14 @@ __device__ __forceinline__ void ld16(const float* p, float (&v)[16])  // p 16-by
 // share a quarter: part `part` takes every nparts-th 16-channel chunk, or
 // for the tail (which needs a pixel's 32 channels together) every
 // nparts-th row.
-template <int BN>
+template <int BN, bool BWD>
 __device__ __forceinline__ void tile_epilogue(const ConvArgs& a, const EpiConsts& ec, uint32_t tmem, int warp, int tid,
                                               int n, int ct, int x0, int y0, int part = 0, int nparts = 1)
 {
     const uint32_t lanebase = tmem + ((uint32_t)(warp * 32) << 16);
     const int x = x0 + tid;
     const bool xin = x < a.W;
-    if (a.epilogue == kEpiTail)
+    if (!BWD && a.epilogue == kEpiTail)
     {
         // BN == Cout == 32: whole pixel in this thread.
         float o[kRows][3];
@@ -343,7 +343,7 @@ __device__ __forceinline__ void tile_epilogue(const ConvArgs& a, const EpiConsts
                 for (int r = 0; r < kRows; ++r) tc::tmem_ld16_take(q[r], v[r]);
             }
             const int cg = ct * BN + c0;  // layer channel of v[.][0]
-            if (a.epilogue <= kEpiUpsample)
+            if (!BWD)
             {
                 // stored through pack8, which rounds to BF16 once; the 2x2 max of the pooled output commutes
                 // with that (monotonic) rounding, so no separate rounding step is needed here
@@ -355,7 +355,7 @@ __device__ __forceinline__ void tile_epilogue(const ConvArgs& a, const EpiConsts
                     for (int j = 0; j < 16; ++j) v[r][j] = act(v[r][j] + bb[j], a.slope);
             }
             const int b0 = (a.out_coff + cg) >> 3;
-            if (a.epilogue >= kEpiBwdMask)
+            if (BWD)
             {
                 bwd_epilogue(a, v, n, y0, x, cg, b0);
             }
@@ -411,7 +411,7 @@ __device__ __forceinline__ void tile_epilogue(const ConvArgs& a, const EpiConsts
     }
 }
 
-template <int BN, int KC, int STAGES>
+template <int BN, int KC, int STAGES, bool BWD>
 __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tmap, ConvArgs a)
 {
     using S = Smem<BN, KC>;
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
     const bool got = tc::mbar_wait(done, 0);
     if (!got && a.err) atomicExch(a.err, 2);
     tc::tc_fence_after();
-    if (got && !s_fail) tile_epilogue<BN>(a, ec, tmem, warp, tid, n, ct, x0, y0);
+    if (got && !s_fail) tile_epilogue<BN, BWD>(a, ec, tmem, warp, tid, n, ct, x0, y0);
 
     tc::tc_fence_before();
     __syncthreads();
@@ -568,8 +568,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
 // ROWS + 2 MMAs per (dx, K step) instead of 3 * ROWS.  The first MMA that
 // reaches an output row (dx = 0, first K step of the first K-block) is
 // issued alone for that row so that it can overwrite instead of add.
-constexpr int kEpiWarps = 8;
-constexpr int kPThreads = 64 + 32 * kEpiWarps;
+constexpr int epi_warps(bool bwd) { return bwd ? 8 : 16; }
+constexpr int pthreads(bool bwd) { return 64 + 32 * epi_warps(bwd); }
 template <int BN, int KC, bool RESW, int ROWS = kRows, int AX = kHaloX>
 struct PSmem
 {
@@ -594,12 +594,13 @@ struct PSmem
 // ones (two thirds of the MMA work, half the rows loaded).  The skip
 // channels' K-blocks run first, as in the DYP kernel, so every output row
 // is initialised before the folded ones accumulate.
-template <int BN, int KC, int STAGES, bool RESW, int ROWS = kRows, bool DYP = false, bool VUP = false>
-__global__ void __launch_bounds__(kPThreads, 1) conv3x3_tc_persistent(const __grid_constant__ CUtensorMap tmap,
+template <int BN, int KC, int STAGES, bool BWD, bool RESW, int ROWS = kRows, bool DYP = false, bool VUP = false>
+__global__ void __launch_bounds__(pthreads(BWD), 1) conv3x3_tc_persistent(const __grid_constant__ CUtensorMap tmap,
                                                                       const __grid_constant__ CUtensorMap tmap2,
                                                                       ConvArgs a)
 {
     static_assert(ROWS == 2 || ROWS == 4 || ROWS == 8, "2-, 4- or 8-row tiles");
+    constexpr int kEpiWarps = epi_warps(BWD), kPThreads = pthreads(BWD);
     static_assert(!DYP || 3 * BN <= 256, "row taps packed into N need 3 * BN <= 256");
     static_assert(!VUP || (DYP && !RESW && ROWS >= 4 && 4 * BN <= 256), "folded upsampling: streamed DYP, 4*BN <= 256");
     // DYP kernels load their A tiles through the chunked view (make_map_chunked)
@@ -888,10 +889,12 @@ __global__ void __launch_bounds__(kPThreads, 1) conv3x3_tc_persistent(const __gr
             tc::tc_fence_after();
             int n, ct, x0, y0;
             coords(t, n, ct, x0, y0);
+            // a quarter's warps share out the 2-row sub-tiles and, within one, its channel chunks
+            constexpr int kSubParts = !BWD && ROWS > 2 ? 2 : 1, kChunkParts = kParts / kSubParts;
 #pragma unroll 1
-            for (int sub = 0; sub < ROWS / 2; ++sub)  // 2-row sub-tiles
-                tile_epilogue<BN>(a, ec, tmem + (uint32_t)b * kAccCols + (uint32_t)(sub * 2 * BN), q, q * 32 + lane,
-                                  n, ct, x0, y0 + 2 * sub, part, kParts);
+            for (int sub = part / kChunkParts; sub < ROWS / 2; sub += kSubParts)
+                tile_epilogue<BN, BWD>(a, ec, tmem + (uint32_t)b * kAccCols + (uint32_t)(sub * 2 * BN), q, q * 32 + lane,
+                                       n, ct, x0, y0 + 2 * sub, part % kChunkParts, kChunkParts);
             tc::tc_fence_before();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&acc_empty[b]);
@@ -989,10 +992,10 @@ cudaError_t launch_dependent(void (*fn)(P...), dim3 grid, int block, int smem, c
     return cudaLaunchKernelEx(&c, fn, std::forward<A>(args)...);
 }
 
-template <int BN, int KC, int STAGES, bool RESW = false, int ROWS = kRows, bool DYP = false, bool VUP = false>
+template <int BN, int KC, int STAGES, bool BWD, bool RESW = false, int ROWS = kRows, bool DYP = false, bool VUP = false>
 cudaError_t launch_persistent(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan& plan)
 {
-    auto fn = conv3x3_tc_persistent<BN, KC, STAGES, RESW, ROWS, DYP, VUP>;
+    auto fn = conv3x3_tc_persistent<BN, KC, STAGES, BWD, RESW, ROWS, DYP, VUP>;
     if (!plan.ready)
     {
         const int KB = a.Cin / KC;
@@ -1029,7 +1032,7 @@ cudaError_t launch_persistent(const __nv_bfloat16* in, const ConvArgs& a, cudaSt
             attr_done = true;
         }
         int per_sm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPThreads, smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, pthreads(BWD), smem);
         if (e != cudaSuccess) return e;
         // TMEM: each CTA holds 2*ROWS*BN of the SM's 512 columns for its lifetime
         const int tmem_fit = 512 / (2 * ROWS * BN);
@@ -1043,10 +1046,10 @@ cudaError_t launch_persistent(const __nv_bfloat16* in, const ConvArgs& a, cudaSt
     }
     ConvArgs b = a;
     b.a_chunked = plan.a_chunked;
-    return launch_dependent(fn, dim3(plan.grid[0]), kPThreads, plan.smem, stream, plan.m, plan.m2, b);
+    return launch_dependent(fn, dim3(plan.grid[0]), pthreads(BWD), plan.smem, stream, plan.m, plan.m2, b);
 }
 
-template <int BN, int KC, int STAGES>
+template <int BN, int KC, int STAGES, bool BWD>
 cudaError_t launch(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan& plan)
 {
     if (!plan.ready)
@@ -1057,7 +1060,7 @@ cudaError_t launch(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stre
         static bool attr_done = false;
         if (!attr_done)
         {
-            e = cudaFuncSetAttribute(conv3x3_tc_kernel<BN, KC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            e = cudaFuncSetAttribute(conv3x3_tc_kernel<BN, KC, STAGES, BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      plan.smem);
             if (e != cudaSuccess) return e;
             attr_done = true;
@@ -1067,7 +1070,7 @@ cudaError_t launch(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stre
         plan.grid[2] = (unsigned)(a.N * (a.Cout / BN));
         plan.ready = true;
     }
-    return launch_dependent(conv3x3_tc_kernel<BN, KC, STAGES>, dim3(plan.grid[0], plan.grid[1], plan.grid[2]), kThreads,
+    return launch_dependent(conv3x3_tc_kernel<BN, KC, STAGES, BWD>, dim3(plan.grid[0], plan.grid[1], plan.grid[2]), kThreads,
                             plan.smem, stream, plan.m, a);
 }
 
@@ -1367,6 +1370,90 @@ cudaError_t conv_pack_many(const ConvPackJob* jobs, int n, cudaStream_t stream)
 }
 
 
+namespace
+{
+// The compiled kernel of a resolved tile (conv3x3_forward).
+template <bool BWD>
+cudaError_t launch_tile(const __nv_bfloat16* in, const ConvArgs& a, const TileCfg& c, cudaStream_t stream, ConvPlan& plan)
+{
+    const int key = c.bn * 1000 + c.kc * 10 + c.stages;
+    if (c.persist == 7)
+        switch (key)
+        {
+        case 32322: return launch_persistent<32, 32, 2, BWD, false, 8, true>(in, a, stream, plan);
+        default: return cudaErrorInvalidValue;
+        }
+    if (c.persist == 6)
+        switch (key)
+        {
+        case 64322: return launch_persistent<64, 32, 2, BWD, false, 4, true>(in, a, stream, plan);
+        case 32323: return launch_persistent<32, 32, 3, BWD, false, 4, true>(in, a, stream, plan);
+        default: return cudaErrorInvalidValue;
+        }
+    if (c.persist == 5)
+        switch (key)
+        {
+        case 32164: return launch_persistent<32, 16, 4, BWD, true, 8, true>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2, BWD, true, 8, true>(in, a, stream, plan);
+        default: return cudaErrorInvalidValue;
+        }
+    if (c.persist == 4)
+        switch (key)
+        {
+        case 32167: return launch_persistent<32, 16, 7, BWD, true, 4, true>(in, a, stream, plan);
+        case 32323: return launch_persistent<32, 32, 3, BWD, true, 4, true>(in, a, stream, plan);
+        case 64322: return launch_persistent<64, 32, 2, BWD, true, 4, true>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, BWD, true, 4, true>(in, a, stream, plan);
+        default: return cudaErrorInvalidValue;
+        }
+    if (c.persist == 3)
+        switch (key)
+        {
+        case 32168: return launch_persistent<32, 16, 8, BWD, true, 4>(in, a, stream, plan);
+        case 32323: return launch_persistent<32, 32, 3, BWD, true, 4>(in, a, stream, plan);
+        case 32324: return launch_persistent<32, 32, 4, BWD, true, 4>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, BWD, true, 4>(in, a, stream, plan);
+        default: return cudaErrorInvalidValue;
+        }
+    if (c.persist == 2)
+        switch (key)
+        {
+        case 32170: return launch_persistent<32, 16, 10, BWD, true>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2, BWD, true>(in, a, stream, plan);
+        case 32325: return launch_persistent<32, 32, 5, BWD, true>(in, a, stream, plan);
+        case 32326: return launch_persistent<32, 32, 6, BWD, true>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, BWD, true>(in, a, stream, plan);
+        case 64324: return launch_persistent<64, 32, 4, BWD, true>(in, a, stream, plan);
+        default: return cudaErrorInvalidValue;
+        }
+    if (c.persist)
+        switch (key)
+        {
+        case 32164: return launch_persistent<32, 16, 4, BWD>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2, BWD>(in, a, stream, plan);
+        case 32324: return launch_persistent<32, 32, 4, BWD>(in, a, stream, plan);
+        case 64164: return launch_persistent<64, 16, 4, BWD>(in, a, stream, plan);
+        case 64322: return launch_persistent<64, 32, 2, BWD>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, BWD>(in, a, stream, plan);
+        case 128163: return launch_persistent<128, 16, 3, BWD>(in, a, stream, plan);
+        case 128322: return launch_persistent<128, 32, 2, BWD>(in, a, stream, plan);
+        default: return cudaErrorInvalidValue;
+        }
+    switch (key)
+    {
+    case 32164: return launch<32, 16, 4, BWD>(in, a, stream, plan);
+    case 32322: return launch<32, 32, 2, BWD>(in, a, stream, plan);
+    case 32324: return launch<32, 32, 4, BWD>(in, a, stream, plan);
+    case 64164: return launch<64, 16, 4, BWD>(in, a, stream, plan);
+    case 64322: return launch<64, 32, 2, BWD>(in, a, stream, plan);
+    case 64323: return launch<64, 32, 3, BWD>(in, a, stream, plan);
+    case 128163: return launch<128, 16, 3, BWD>(in, a, stream, plan);
+    case 128322: return launch<128, 32, 2, BWD>(in, a, stream, plan);
+    }
+    return cudaErrorInvalidValue;
+}
+}  // namespace
+
 cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan* kept)
 {
     if (a.Cin % 16 != 0 || (a.Cout != 32 && a.Cout != 64 && a.Cout != 128 && a.Cout != 256)) return cudaErrorInvalidValue;
@@ -1392,6 +1479,7 @@ cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStre
     k.Cout = a.Cout;
     k.up_C = a.up_C;
     k.tile = c;
+    k.bwd = a.epilogue >= kEpiBwdMask;
     if (std::memcmp(&k, &plan.key, sizeof k) != 0)
     {
         plan.ready = false;
@@ -1400,84 +1488,11 @@ cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStre
     if (a.up_C > 0)
     {
         if (!conv_tile_folds(c, a.Cin, a.Cout, a.up_C)) return cudaErrorInvalidValue;
-        if (c.persist == 7) return launch_persistent<32, 32, 2, false, 8, true, true>(in, a, stream, plan);
-        if (key == 64322) return launch_persistent<64, 32, 2, false, 4, true, true>(in, a, stream, plan);
-        return launch_persistent<32, 32, 3, false, 4, true, true>(in, a, stream, plan);
+        if (c.persist == 7) return launch_persistent<32, 32, 2, false, false, 8, true, true>(in, a, stream, plan);
+        if (key == 64322) return launch_persistent<64, 32, 2, false, false, 4, true, true>(in, a, stream, plan);
+        return launch_persistent<32, 32, 3, false, false, 4, true, true>(in, a, stream, plan);
     }
-    if (c.persist == 7)
-        switch (key)
-        {
-        case 32322: return launch_persistent<32, 32, 2, false, 8, true>(in, a, stream, plan);
-        default: return cudaErrorInvalidValue;
-        }
-    if (c.persist == 6)
-        switch (key)
-        {
-        case 64322: return launch_persistent<64, 32, 2, false, 4, true>(in, a, stream, plan);
-        case 32323: return launch_persistent<32, 32, 3, false, 4, true>(in, a, stream, plan);
-        default: return cudaErrorInvalidValue;
-        }
-    if (c.persist == 5)
-        switch (key)
-        {
-        case 32164: return launch_persistent<32, 16, 4, true, 8, true>(in, a, stream, plan);
-        case 32322: return launch_persistent<32, 32, 2, true, 8, true>(in, a, stream, plan);
-        default: return cudaErrorInvalidValue;
-        }
-    if (c.persist == 4)
-        switch (key)
-        {
-        case 32167: return launch_persistent<32, 16, 7, true, 4, true>(in, a, stream, plan);
-        case 32323: return launch_persistent<32, 32, 3, true, 4, true>(in, a, stream, plan);
-        case 64322: return launch_persistent<64, 32, 2, true, 4, true>(in, a, stream, plan);
-        case 64323: return launch_persistent<64, 32, 3, true, 4, true>(in, a, stream, plan);
-        default: return cudaErrorInvalidValue;
-        }
-    if (c.persist == 3)
-        switch (key)
-        {
-        case 32168: return launch_persistent<32, 16, 8, true, 4>(in, a, stream, plan);
-        case 32323: return launch_persistent<32, 32, 3, true, 4>(in, a, stream, plan);
-        case 32324: return launch_persistent<32, 32, 4, true, 4>(in, a, stream, plan);
-        case 64323: return launch_persistent<64, 32, 3, true, 4>(in, a, stream, plan);
-        default: return cudaErrorInvalidValue;
-        }
-    if (c.persist == 2)
-        switch (key)
-        {
-        case 32170: return launch_persistent<32, 16, 10, true>(in, a, stream, plan);
-        case 32322: return launch_persistent<32, 32, 2, true>(in, a, stream, plan);
-        case 32325: return launch_persistent<32, 32, 5, true>(in, a, stream, plan);
-        case 32326: return launch_persistent<32, 32, 6, true>(in, a, stream, plan);
-        case 64323: return launch_persistent<64, 32, 3, true>(in, a, stream, plan);
-        case 64324: return launch_persistent<64, 32, 4, true>(in, a, stream, plan);
-        default: return cudaErrorInvalidValue;
-        }
-    if (c.persist)
-        switch (key)
-        {
-        case 32164: return launch_persistent<32, 16, 4>(in, a, stream, plan);
-        case 32322: return launch_persistent<32, 32, 2>(in, a, stream, plan);
-        case 32324: return launch_persistent<32, 32, 4>(in, a, stream, plan);
-        case 64164: return launch_persistent<64, 16, 4>(in, a, stream, plan);
-        case 64322: return launch_persistent<64, 32, 2>(in, a, stream, plan);
-        case 64323: return launch_persistent<64, 32, 3>(in, a, stream, plan);
-        case 128163: return launch_persistent<128, 16, 3>(in, a, stream, plan);
-        case 128322: return launch_persistent<128, 32, 2>(in, a, stream, plan);
-        default: return cudaErrorInvalidValue;
-        }
-    switch (key)
-    {
-    case 32164: return launch<32, 16, 4>(in, a, stream, plan);
-    case 32322: return launch<32, 32, 2>(in, a, stream, plan);
-    case 32324: return launch<32, 32, 4>(in, a, stream, plan);
-    case 64164: return launch<64, 16, 4>(in, a, stream, plan);
-    case 64322: return launch<64, 32, 2>(in, a, stream, plan);
-    case 64323: return launch<64, 32, 3>(in, a, stream, plan);
-    case 128163: return launch<128, 16, 3>(in, a, stream, plan);
-    case 128322: return launch<128, 32, 2>(in, a, stream, plan);
-    }
-    return cudaErrorInvalidValue;
+    return a.epilogue >= kEpiBwdMask ? launch_tile<true>(in, a, c, stream, plan) : launch_tile<false>(in, a, c, stream, plan);
 }
 
 cudaError_t to_blocked_bf16(const float* x, int N, int C, int H, int W, __nv_bfloat16* out, int Cpad,
