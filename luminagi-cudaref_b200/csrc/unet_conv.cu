@@ -70,6 +70,14 @@ struct Smem
     static constexpr int kStage = ((kABytes + kBBytes + 1023) / 1024) * 1024;
 };
 
+// The epilogues a kernel is compiled with: a kernel that carries all of them has the registers of the largest
+// (unpooling reads four windows of 16 channels), which leaves too few for the sixteen epilogue warps.
+constexpr int kEpiClassForward = 0, kEpiClassBackward = 1, kEpiClassUnpool = 2;
+constexpr int epi_class(int epilogue)
+{
+    return epilogue < kEpiBwdMask ? kEpiClassForward : (epilogue == kEpiBwdUnpool ? kEpiClassUnpool : kEpiClassBackward);
+}
+
 __device__ __forceinline__ float act(float v, float slope) { return v > 0.0f ? v : v * slope; }
 
 __device__ __forceinline__ uint4 pack8(const float* v)
@@ -116,12 +124,13 @@ __device__ __forceinline__ float dact(float y, float slope) { return y > 0.0f ? 
 
 // Input-gradient epilogues (see ConvEpilogue).  v[r][j]: gradient of conv
 // input channel cg+j at (y0+r, x) of this (backward) convolution.
+template <int EPI>
 __device__ __forceinline__ void bwd_epilogue(const ConvArgs& a, float (&v)[kRows][16], int n, int y0, int x, int cg,
                                              int b0)
 {
     const bool xin = x < a.W;
     const int rb = (a.ref_coff + cg) >> 3;
-    if (a.epilogue == kEpiBwdMask || a.epilogue == kEpiBwdStore)
+    if (EPI == kEpiClassBackward && (a.epilogue == kEpiBwdMask || a.epilogue == kEpiBwdStore))
     {
 #pragma unroll
         for (int r = 0; r < kRows; ++r)
@@ -145,7 +154,7 @@ __device__ __forceinline__ void bwd_epilogue(const ConvArgs& a, float (&v)[kRows
             *blk(a.out, a.out_C, a.H, a.W, n, b0 + 1, y, x) = pack8(o + 8);
         }
     }
-    else if (a.epilogue == kEpiBwdSumPool)
+    else if (EPI == kEpiClassBackward)  // kEpiBwdSumPool
     {
         // Gradient of a nearest 2x upsample: sum of the 2x2 children.
         float s[16];
@@ -251,14 +260,14 @@ __device__ __forceinline__ void ld16(const float* p, float (&v)[16])  // p 16-by
 // share a quarter: part `part` takes every nparts-th 16-channel chunk, or
 // for the tail (which needs a pixel's 32 channels together) every
 // nparts-th row.
-template <int BN, bool BWD>
+template <int BN, int EPI>
 __device__ __forceinline__ void tile_epilogue(const ConvArgs& a, const EpiConsts& ec, uint32_t tmem, int warp, int tid,
                                               int n, int ct, int x0, int y0, int part = 0, int nparts = 1)
 {
     const uint32_t lanebase = tmem + ((uint32_t)(warp * 32) << 16);
     const int x = x0 + tid;
     const bool xin = x < a.W;
-    if (!BWD && a.epilogue == kEpiTail)
+    if (EPI == kEpiClassForward && a.epilogue == kEpiTail)
     {
         // BN == Cout == 32: whole pixel in this thread.
         float o[kRows][3];
@@ -343,7 +352,7 @@ __device__ __forceinline__ void tile_epilogue(const ConvArgs& a, const EpiConsts
                 for (int r = 0; r < kRows; ++r) tc::tmem_ld16_take(q[r], v[r]);
             }
             const int cg = ct * BN + c0;  // layer channel of v[.][0]
-            if (!BWD)
+            if (EPI == kEpiClassForward)
             {
                 // stored through pack8, which rounds to BF16 once; the 2x2 max of the pooled output commutes
                 // with that (monotonic) rounding, so no separate rounding step is needed here
@@ -355,9 +364,9 @@ __device__ __forceinline__ void tile_epilogue(const ConvArgs& a, const EpiConsts
                     for (int j = 0; j < 16; ++j) v[r][j] = act(v[r][j] + bb[j], a.slope);
             }
             const int b0 = (a.out_coff + cg) >> 3;
-            if (BWD)
+            if (EPI != kEpiClassForward)
             {
-                bwd_epilogue(a, v, n, y0, x, cg, b0);
+                bwd_epilogue<EPI>(a, v, n, y0, x, cg, b0);
             }
             else if (a.epilogue == kEpiStore)
             {
@@ -411,7 +420,7 @@ __device__ __forceinline__ void tile_epilogue(const ConvArgs& a, const EpiConsts
     }
 }
 
-template <int BN, int KC, int STAGES, bool BWD>
+template <int BN, int KC, int STAGES, int EPI>
 __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tmap, ConvArgs a)
 {
     using S = Smem<BN, KC>;
@@ -522,7 +531,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
     const bool got = tc::mbar_wait(done, 0);
     if (!got && a.err) atomicExch(a.err, 2);
     tc::tc_fence_after();
-    if (got && !s_fail) tile_epilogue<BN, BWD>(a, ec, tmem, warp, tid, n, ct, x0, y0);
+    if (got && !s_fail) tile_epilogue<BN, EPI>(a, ec, tmem, warp, tid, n, ct, x0, y0);
 
     tc::tc_fence_before();
     __syncthreads();
@@ -568,8 +577,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
 // ROWS + 2 MMAs per (dx, K step) instead of 3 * ROWS.  The first MMA that
 // reaches an output row (dx = 0, first K step of the first K-block) is
 // issued alone for that row so that it can overwrite instead of add.
-constexpr int epi_warps(bool bwd) { return bwd ? 8 : 16; }
-constexpr int pthreads(bool bwd) { return 64 + 32 * epi_warps(bwd); }
+constexpr int epi_warps(int epi) { return epi == kEpiClassUnpool ? 8 : 16; }
+constexpr int pthreads(int epi) { return 64 + 32 * epi_warps(epi); }
 template <int BN, int KC, bool RESW, int ROWS = kRows, int AX = kHaloX>
 struct PSmem
 {
@@ -594,13 +603,13 @@ struct PSmem
 // ones (two thirds of the MMA work, half the rows loaded).  The skip
 // channels' K-blocks run first, as in the DYP kernel, so every output row
 // is initialised before the folded ones accumulate.
-template <int BN, int KC, int STAGES, bool BWD, bool RESW, int ROWS = kRows, bool DYP = false, bool VUP = false>
-__global__ void __launch_bounds__(pthreads(BWD), 1) conv3x3_tc_persistent(const __grid_constant__ CUtensorMap tmap,
+template <int BN, int KC, int STAGES, int EPI, bool RESW, int ROWS = kRows, bool DYP = false, bool VUP = false>
+__global__ void __launch_bounds__(pthreads(EPI), 1) conv3x3_tc_persistent(const __grid_constant__ CUtensorMap tmap,
                                                                       const __grid_constant__ CUtensorMap tmap2,
                                                                       ConvArgs a)
 {
     static_assert(ROWS == 2 || ROWS == 4 || ROWS == 8, "2-, 4- or 8-row tiles");
-    constexpr int kEpiWarps = epi_warps(BWD), kPThreads = pthreads(BWD);
+    constexpr int kEpiWarps = epi_warps(EPI), kPThreads = pthreads(EPI);
     static_assert(!DYP || 3 * BN <= 256, "row taps packed into N need 3 * BN <= 256");
     static_assert(!VUP || (DYP && !RESW && ROWS >= 4 && 4 * BN <= 256), "folded upsampling: streamed DYP, 4*BN <= 256");
     // DYP kernels load their A tiles through the chunked view (make_map_chunked)
@@ -890,10 +899,10 @@ __global__ void __launch_bounds__(pthreads(BWD), 1) conv3x3_tc_persistent(const 
             int n, ct, x0, y0;
             coords(t, n, ct, x0, y0);
             // a quarter's warps share out the 2-row sub-tiles and, within one, its channel chunks
-            constexpr int kSubParts = !BWD && ROWS > 2 ? 2 : 1, kChunkParts = kParts / kSubParts;
+            constexpr int kSubParts = EPI != kEpiClassUnpool && ROWS > 2 ? 2 : 1, kChunkParts = kParts / kSubParts;
 #pragma unroll 1
             for (int sub = part / kChunkParts; sub < ROWS / 2; sub += kSubParts)
-                tile_epilogue<BN, BWD>(a, ec, tmem + (uint32_t)b * kAccCols + (uint32_t)(sub * 2 * BN), q, q * 32 + lane,
+                tile_epilogue<BN, EPI>(a, ec, tmem + (uint32_t)b * kAccCols + (uint32_t)(sub * 2 * BN), q, q * 32 + lane,
                                        n, ct, x0, y0 + 2 * sub, part % kChunkParts, kChunkParts);
             tc::tc_fence_before();
             __syncwarp();
@@ -992,10 +1001,10 @@ cudaError_t launch_dependent(void (*fn)(P...), dim3 grid, int block, int smem, c
     return cudaLaunchKernelEx(&c, fn, std::forward<A>(args)...);
 }
 
-template <int BN, int KC, int STAGES, bool BWD, bool RESW = false, int ROWS = kRows, bool DYP = false, bool VUP = false>
+template <int BN, int KC, int STAGES, int EPI, bool RESW = false, int ROWS = kRows, bool DYP = false, bool VUP = false>
 cudaError_t launch_persistent(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan& plan)
 {
-    auto fn = conv3x3_tc_persistent<BN, KC, STAGES, BWD, RESW, ROWS, DYP, VUP>;
+    auto fn = conv3x3_tc_persistent<BN, KC, STAGES, EPI, RESW, ROWS, DYP, VUP>;
     if (!plan.ready)
     {
         const int KB = a.Cin / KC;
@@ -1032,7 +1041,7 @@ cudaError_t launch_persistent(const __nv_bfloat16* in, const ConvArgs& a, cudaSt
             attr_done = true;
         }
         int per_sm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, pthreads(BWD), smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, pthreads(EPI), smem);
         if (e != cudaSuccess) return e;
         // TMEM: each CTA holds 2*ROWS*BN of the SM's 512 columns for its lifetime
         const int tmem_fit = 512 / (2 * ROWS * BN);
@@ -1046,10 +1055,10 @@ cudaError_t launch_persistent(const __nv_bfloat16* in, const ConvArgs& a, cudaSt
     }
     ConvArgs b = a;
     b.a_chunked = plan.a_chunked;
-    return launch_dependent(fn, dim3(plan.grid[0]), pthreads(BWD), plan.smem, stream, plan.m, plan.m2, b);
+    return launch_dependent(fn, dim3(plan.grid[0]), pthreads(EPI), plan.smem, stream, plan.m, plan.m2, b);
 }
 
-template <int BN, int KC, int STAGES, bool BWD>
+template <int BN, int KC, int STAGES, int EPI>
 cudaError_t launch(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan& plan)
 {
     if (!plan.ready)
@@ -1060,7 +1069,7 @@ cudaError_t launch(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stre
         static bool attr_done = false;
         if (!attr_done)
         {
-            e = cudaFuncSetAttribute(conv3x3_tc_kernel<BN, KC, STAGES, BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            e = cudaFuncSetAttribute(conv3x3_tc_kernel<BN, KC, STAGES, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      plan.smem);
             if (e != cudaSuccess) return e;
             attr_done = true;
@@ -1070,7 +1079,7 @@ cudaError_t launch(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stre
         plan.grid[2] = (unsigned)(a.N * (a.Cout / BN));
         plan.ready = true;
     }
-    return launch_dependent(conv3x3_tc_kernel<BN, KC, STAGES, BWD>, dim3(plan.grid[0], plan.grid[1], plan.grid[2]), kThreads,
+    return launch_dependent(conv3x3_tc_kernel<BN, KC, STAGES, EPI>, dim3(plan.grid[0], plan.grid[1], plan.grid[2]), kThreads,
                             plan.smem, stream, plan.m, a);
 }
 
@@ -1373,82 +1382,82 @@ cudaError_t conv_pack_many(const ConvPackJob* jobs, int n, cudaStream_t stream)
 namespace
 {
 // The compiled kernel of a resolved tile (conv3x3_forward).
-template <bool BWD>
+template <int EPI>
 cudaError_t launch_tile(const __nv_bfloat16* in, const ConvArgs& a, const TileCfg& c, cudaStream_t stream, ConvPlan& plan)
 {
     const int key = c.bn * 1000 + c.kc * 10 + c.stages;
     if (c.persist == 7)
         switch (key)
         {
-        case 32322: return launch_persistent<32, 32, 2, BWD, false, 8, true>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2, EPI, false, 8, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 6)
         switch (key)
         {
-        case 64322: return launch_persistent<64, 32, 2, BWD, false, 4, true>(in, a, stream, plan);
-        case 32323: return launch_persistent<32, 32, 3, BWD, false, 4, true>(in, a, stream, plan);
+        case 64322: return launch_persistent<64, 32, 2, EPI, false, 4, true>(in, a, stream, plan);
+        case 32323: return launch_persistent<32, 32, 3, EPI, false, 4, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 5)
         switch (key)
         {
-        case 32164: return launch_persistent<32, 16, 4, BWD, true, 8, true>(in, a, stream, plan);
-        case 32322: return launch_persistent<32, 32, 2, BWD, true, 8, true>(in, a, stream, plan);
+        case 32164: return launch_persistent<32, 16, 4, EPI, true, 8, true>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2, EPI, true, 8, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 4)
         switch (key)
         {
-        case 32167: return launch_persistent<32, 16, 7, BWD, true, 4, true>(in, a, stream, plan);
-        case 32323: return launch_persistent<32, 32, 3, BWD, true, 4, true>(in, a, stream, plan);
-        case 64322: return launch_persistent<64, 32, 2, BWD, true, 4, true>(in, a, stream, plan);
-        case 64323: return launch_persistent<64, 32, 3, BWD, true, 4, true>(in, a, stream, plan);
+        case 32167: return launch_persistent<32, 16, 7, EPI, true, 4, true>(in, a, stream, plan);
+        case 32323: return launch_persistent<32, 32, 3, EPI, true, 4, true>(in, a, stream, plan);
+        case 64322: return launch_persistent<64, 32, 2, EPI, true, 4, true>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, EPI, true, 4, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 3)
         switch (key)
         {
-        case 32168: return launch_persistent<32, 16, 8, BWD, true, 4>(in, a, stream, plan);
-        case 32323: return launch_persistent<32, 32, 3, BWD, true, 4>(in, a, stream, plan);
-        case 32324: return launch_persistent<32, 32, 4, BWD, true, 4>(in, a, stream, plan);
-        case 64323: return launch_persistent<64, 32, 3, BWD, true, 4>(in, a, stream, plan);
+        case 32168: return launch_persistent<32, 16, 8, EPI, true, 4>(in, a, stream, plan);
+        case 32323: return launch_persistent<32, 32, 3, EPI, true, 4>(in, a, stream, plan);
+        case 32324: return launch_persistent<32, 32, 4, EPI, true, 4>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, EPI, true, 4>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist == 2)
         switch (key)
         {
-        case 32170: return launch_persistent<32, 16, 10, BWD, true>(in, a, stream, plan);
-        case 32322: return launch_persistent<32, 32, 2, BWD, true>(in, a, stream, plan);
-        case 32325: return launch_persistent<32, 32, 5, BWD, true>(in, a, stream, plan);
-        case 32326: return launch_persistent<32, 32, 6, BWD, true>(in, a, stream, plan);
-        case 64323: return launch_persistent<64, 32, 3, BWD, true>(in, a, stream, plan);
-        case 64324: return launch_persistent<64, 32, 4, BWD, true>(in, a, stream, plan);
+        case 32170: return launch_persistent<32, 16, 10, EPI, true>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2, EPI, true>(in, a, stream, plan);
+        case 32325: return launch_persistent<32, 32, 5, EPI, true>(in, a, stream, plan);
+        case 32326: return launch_persistent<32, 32, 6, EPI, true>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, EPI, true>(in, a, stream, plan);
+        case 64324: return launch_persistent<64, 32, 4, EPI, true>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     if (c.persist)
         switch (key)
         {
-        case 32164: return launch_persistent<32, 16, 4, BWD>(in, a, stream, plan);
-        case 32322: return launch_persistent<32, 32, 2, BWD>(in, a, stream, plan);
-        case 32324: return launch_persistent<32, 32, 4, BWD>(in, a, stream, plan);
-        case 64164: return launch_persistent<64, 16, 4, BWD>(in, a, stream, plan);
-        case 64322: return launch_persistent<64, 32, 2, BWD>(in, a, stream, plan);
-        case 64323: return launch_persistent<64, 32, 3, BWD>(in, a, stream, plan);
-        case 128163: return launch_persistent<128, 16, 3, BWD>(in, a, stream, plan);
-        case 128322: return launch_persistent<128, 32, 2, BWD>(in, a, stream, plan);
+        case 32164: return launch_persistent<32, 16, 4, EPI>(in, a, stream, plan);
+        case 32322: return launch_persistent<32, 32, 2, EPI>(in, a, stream, plan);
+        case 32324: return launch_persistent<32, 32, 4, EPI>(in, a, stream, plan);
+        case 64164: return launch_persistent<64, 16, 4, EPI>(in, a, stream, plan);
+        case 64322: return launch_persistent<64, 32, 2, EPI>(in, a, stream, plan);
+        case 64323: return launch_persistent<64, 32, 3, EPI>(in, a, stream, plan);
+        case 128163: return launch_persistent<128, 16, 3, EPI>(in, a, stream, plan);
+        case 128322: return launch_persistent<128, 32, 2, EPI>(in, a, stream, plan);
         default: return cudaErrorInvalidValue;
         }
     switch (key)
     {
-    case 32164: return launch<32, 16, 4, BWD>(in, a, stream, plan);
-    case 32322: return launch<32, 32, 2, BWD>(in, a, stream, plan);
-    case 32324: return launch<32, 32, 4, BWD>(in, a, stream, plan);
-    case 64164: return launch<64, 16, 4, BWD>(in, a, stream, plan);
-    case 64322: return launch<64, 32, 2, BWD>(in, a, stream, plan);
-    case 64323: return launch<64, 32, 3, BWD>(in, a, stream, plan);
-    case 128163: return launch<128, 16, 3, BWD>(in, a, stream, plan);
-    case 128322: return launch<128, 32, 2, BWD>(in, a, stream, plan);
+    case 32164: return launch<32, 16, 4, EPI>(in, a, stream, plan);
+    case 32322: return launch<32, 32, 2, EPI>(in, a, stream, plan);
+    case 32324: return launch<32, 32, 4, EPI>(in, a, stream, plan);
+    case 64164: return launch<64, 16, 4, EPI>(in, a, stream, plan);
+    case 64322: return launch<64, 32, 2, EPI>(in, a, stream, plan);
+    case 64323: return launch<64, 32, 3, EPI>(in, a, stream, plan);
+    case 128163: return launch<128, 16, 3, EPI>(in, a, stream, plan);
+    case 128322: return launch<128, 32, 2, EPI>(in, a, stream, plan);
     }
     return cudaErrorInvalidValue;
 }
@@ -1479,7 +1488,7 @@ cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStre
     k.Cout = a.Cout;
     k.up_C = a.up_C;
     k.tile = c;
-    k.bwd = a.epilogue >= kEpiBwdMask;
+    k.epi = epi_class(a.epilogue);
     if (std::memcmp(&k, &plan.key, sizeof k) != 0)
     {
         plan.ready = false;
@@ -1488,11 +1497,16 @@ cudaError_t conv3x3_forward(const __nv_bfloat16* in, const ConvArgs& a, cudaStre
     if (a.up_C > 0)
     {
         if (!conv_tile_folds(c, a.Cin, a.Cout, a.up_C)) return cudaErrorInvalidValue;
-        if (c.persist == 7) return launch_persistent<32, 32, 2, false, false, 8, true, true>(in, a, stream, plan);
-        if (key == 64322) return launch_persistent<64, 32, 2, false, false, 4, true, true>(in, a, stream, plan);
-        return launch_persistent<32, 32, 3, false, false, 4, true, true>(in, a, stream, plan);
+        if (c.persist == 7) return launch_persistent<32, 32, 2, kEpiClassForward, false, 8, true, true>(in, a, stream, plan);
+        if (key == 64322) return launch_persistent<64, 32, 2, kEpiClassForward, false, 4, true, true>(in, a, stream, plan);
+        return launch_persistent<32, 32, 3, kEpiClassForward, false, 4, true, true>(in, a, stream, plan);
     }
-    return a.epilogue >= kEpiBwdMask ? launch_tile<true>(in, a, c, stream, plan) : launch_tile<false>(in, a, c, stream, plan);
+    switch (k.epi)
+    {
+    case kEpiClassForward: return launch_tile<kEpiClassForward>(in, a, c, stream, plan);
+    case kEpiClassBackward: return launch_tile<kEpiClassBackward>(in, a, c, stream, plan);
+    default: return launch_tile<kEpiClassUnpool>(in, a, c, stream, plan);
+    }
 }
 
 cudaError_t to_blocked_bf16(const float* x, int N, int C, int H, int W, __nv_bfloat16* out, int Cpad,

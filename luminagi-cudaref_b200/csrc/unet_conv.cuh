@@ -124,7 +124,7 @@ struct ConvPlan
     struct Key
     {
         const void *in, *up_h;
-        int N, H, W, Cin, Cout, up_C, bwd;
+        int N, H, W, Cin, Cout, up_C, epi;
         ConvTile tile;
     } key{};
     bool ready = false;
