@@ -118,6 +118,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
+// The same descriptor moved by `bytes` (a multiple of 16).  Shared memory ends below 2^14 * 16 bytes, so the
+// address field takes the sum without a carry.
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes)
+{
+    return (desc & 0xffffffff00000000ull) | (uint32_t)((uint32_t)desc + (bytes >> 4));
+}
 // Instruction descriptor for kind::f16: BF16 x BF16 -> FP32, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N)
 {

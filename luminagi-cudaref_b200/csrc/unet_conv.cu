@@ -630,7 +630,8 @@ __global__ void __launch_bounds__(pthreads(EPI), 1) conv3x3_tc_persistent(const 
     __shared__ volatile int s_fail;
     __shared__ EpiConsts ec;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the warp's number by way of a shuffle: the same in all lanes, for the branches on it
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int n_cot = a.Cout / BN;
     const int tiles_x = (a.W + kTileX - 1) / kTileX, tiles_y = (a.H + ROWS - 1) / ROWS;
     const int n_tiles = tiles_x * tiles_y * a.N * n_cot;
@@ -692,7 +693,8 @@ __global__ void __launch_bounds__(pthreads(EPI), 1) conv3x3_tc_persistent(const 
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const uint32_t smem0 = tc::smem_u32(smem), wres0 = tc::smem_u32(wres);
 
     if (warp == 0)
     {
@@ -752,134 +754,140 @@ __global__ void __launch_bounds__(pthreads(EPI), 1) conv3x3_tc_persistent(const 
     }
     else if (warp == 1)
     {
-        if (lane == 0)
+        // All lanes walk the loops, so that loop state and descriptors are the same in the whole warp, lane 0 issues,
+        // and a descriptor is the stage's own plus an offset instead of built anew for each MMA.  Both together,
+        // against lane 0 alone building each one: 622 -> 611 us a pass at 1x864x1728, 550 -> 541 (HDR, 1x720x1280),
+        // 4.71 -> 4.66 ms at 8x864x1728, 157.2 -> 155.5 us at 1x128x128, 178.6 -> 178.6 at 1x256x512 with 12
+        // channels.  What each of the two gives was not measured apart.
+        const bool leader = lane == 0;
+        int it = 0, j = 0;
+        if (RESW && !tc::mbar_wait(wfull, 0) && leader) fail(5);
+        for (int t = blockIdx.x; t < n_tiles && !s_fail; t += gridDim.x, ++j)
         {
-            int it = 0, j = 0;
-            if (RESW && !tc::mbar_wait(wfull, 0)) fail(5);
-            for (int t = blockIdx.x; t < n_tiles && !s_fail; t += gridDim.x, ++j)
+            const int b = j & 1, v = j >> 1;
+            if (v > 0 && !tc::mbar_wait(&acc_empty[b], (uint32_t)((v - 1) & 1)))
             {
-                const int b = j & 1, v = j >> 1;
-                if (v > 0 && !tc::mbar_wait(&acc_empty[b], (uint32_t)((v - 1) & 1)))
+                if (leader) fail(4);
+                break;
+            }
+            tc::tc_fence_after();
+            const uint32_t acc = tmem + (uint32_t)b * kAccCols;
+            bool ok = true;
+            for (int kb = 0; kb < KB; ++kb, ++it)
+            {
+                const int s = it % STAGES;
+                if (!tc::mbar_wait(&full[s], (uint32_t)((it / STAGES) & 1)))
                 {
-                    fail(4);
+                    ok = false;
                     break;
                 }
                 tc::tc_fence_after();
-                const uint32_t acc = tmem + (uint32_t)b * kAccCols;
-                bool ok = true;
-                for (int kb = 0; kb < KB; ++kb, ++it)
+                const uint32_t abase = smem0 + (uint32_t)(s * P::kStage);
+                const uint32_t bbase = RESW ? wres0 + (uint32_t)(kb * S::kBBytes) : abase + (uint32_t)S::kABytes;
+                if (VUP && kb >= KBS)
                 {
-                    const int s = it % STAGES;
-                    if (!tc::mbar_wait(&full[s], (uint32_t)((it / STAGES) & 1)))
-                    {
-                        ok = false;
-                        break;
-                    }
-                    tc::tc_fence_after();
-                    const uint32_t abase = tc::smem_u32(smem + s * P::kStage);
-                    const uint32_t bbase =
-                        RESW ? tc::smem_u32(wres) + (uint32_t)(kb * S::kBBytes) : abase + (uint32_t)S::kABytes;
-                    if (VUP && kb >= KBS)
-                    {
-                        // folded K-block: weights [dx][KC/8][ky2 | ky1+ky2 | ky0+ky1 | ky0][BN][8]; low-resolution
-                        // row h of the tile reaches output rows 2h-3+s (slot s) of those inside the tile
-                        const uint32_t ubase = abase + kAUBytes;
+                    // folded K-block: weights [dx][KC/8][ky2 | ky1+ky2 | ky0+ky1 | ky0][BN][8]; low-resolution
+                    // row h of the tile reaches output rows 2h-3+s (slot s) of those inside the tile
+                    const uint64_t ad0 = tc::smem_desc(abase + AX0 * 16, kLboAU, 128);
+                    const uint64_t bd0 = tc::smem_desc(abase + kAUBytes, kLboBU, 128);
 #pragma unroll 1
-                        for (int h = 0; h < kRowsU; ++h)
-                        {
-                            const int smin = h == 0 ? 3 : (h == 1 ? 1 : 0);
-                            const int smax = ROWS + 2 - 2 * h < 3 ? ROWS + 2 - 2 * h : 3;
-                            const int nb = smax - smin + 1;
-                            const uint32_t id = nb == 4 ? kIdesc4 : nb == 3 ? kIdesc3 : (nb == 2 ? kIdesc2 : kIdesc);
-                            const uint32_t dcol = acc + (uint32_t)((2 * h - 3 + smin) * BN);
-#pragma unroll
-                            for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-                                for (int ks = 0; ks < KC / 16; ++ks)
-                                {
-                                    const uint32_t aoff =
-                                        (uint32_t)(2 * ks) * kLboAU + (uint32_t)((h * AX + AX0 + dx) * 16);
-                                    const uint64_t ad = tc::smem_desc(abase + aoff, kLboAU, 128);
-                                    const uint32_t plane = ubase + (uint32_t)((dx * (KC / 8) + 2 * ks) * kLboBU);
-                                    const uint64_t bd =
-                                        tc::smem_desc(plane + (uint32_t)(smin * BN * 16), kLboBU, 128);
-                                    tc::mma_bf16(dcol, ad, bd, id, 1u);
-                                }
-                        }
-                    }
-                    else if (DYP)
+                    for (int h = 0; h < kRowsU; ++h)
                     {
-                        // weights of K-block kb: [dx][KC/8][dy = 2, 1, 0][BN][8]
-#pragma unroll 1
-                        for (int h = 0; h < ROWS + 2; ++h)
-                        {
-                            const int dmax = h < 2 ? h : 2;                        // the row taps whose output
-                            const int dmin = h - ROWS + 1 > 0 ? h - ROWS + 1 : 0;  // row h - dy is in the tile
-                            const int nb = dmax - dmin + 1;
-                            const uint32_t id = nb == 3 ? kIdesc3 : (nb == 2 ? kIdesc2 : kIdesc);
-                            const uint32_t dcol = acc + (uint32_t)((h - dmax) * BN);
-                            const bool first = kb == 0 && dmin == 0;  // output row h starts here
+                        const int smin = h == 0 ? 3 : (h == 1 ? 1 : 0);
+                        const int smax = ROWS + 2 - 2 * h < 3 ? ROWS + 2 - 2 * h : 3;
+                        const int nb = smax - smin + 1;
+                        const uint32_t id = nb == 4 ? kIdesc4 : nb == 3 ? kIdesc3 : (nb == 2 ? kIdesc2 : kIdesc);
+                        const uint32_t dcol = acc + (uint32_t)((2 * h - 3 + smin) * BN);
+                        const uint64_t adh = tc::desc_at(ad0, (uint32_t)(h * AX * 16));
+                        const uint64_t bdh = tc::desc_at(bd0, (uint32_t)(smin * BN * 16));
 #pragma unroll
-                            for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-                                for (int ks = 0; ks < KC / 16; ++ks)
-                                {
-                                    const uint32_t aoff =
-                                        (uint32_t)(2 * ks) * kLboA + (uint32_t)((h * AX + AX0 + dx) * 16);
-                                    const uint64_t ad = tc::smem_desc(abase + aoff, kLboA, 128);
-                                    const uint32_t plane = bbase + (uint32_t)((dx * (KC / 8) + 2 * ks) * kLboB);
-                                    const uint64_t bd =
-                                        tc::smem_desc(plane + (uint32_t)((2 - dmax) * BN * 16), kLboB, 128);
-                                    if (first && dx == 0 && ks == 0)
-                                    {
-                                        tc::mma_bf16(acc + (uint32_t)(h * BN), ad,
-                                                     tc::smem_desc(plane + 2 * BN * 16, kLboB, 128), kIdesc, 0u);
-                                        if (dmax > 0) tc::mma_bf16(dcol, ad, bd, dmax == 2 ? kIdesc2 : kIdesc, 1u);
-                                    }
-                                    else
-                                        tc::mma_bf16(dcol, ad, bd, id, 1u);
-                                }
-                        }
-                    }
-                    else
-                    {
-#pragma unroll 1
-                        for (int tap = 0; tap < 9; ++tap)
-                        {
-                            const int dy = tap / 3, dx = tap % 3;
+                        for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
                             for (int ks = 0; ks < KC / 16; ++ks)
                             {
-                                const uint64_t bd = tc::smem_desc(
-                                    bbase + (uint32_t)((tap * (KC / 8) + 2 * ks) * BN * 16), kLboB, 128);
+                                const uint64_t ad = tc::desc_at(adh, (uint32_t)(2 * ks) * kLboAU + (uint32_t)(dx * 16));
+                                const uint64_t bd = tc::desc_at(bdh, (uint32_t)((dx * (KC / 8) + 2 * ks) * kLboBU));
+                                if (leader) tc::mma_bf16(dcol, ad, bd, id, 1u);
+                            }
+                    }
+                }
+                else if (DYP)
+                {
+                    // weights of K-block kb: [dx][KC/8][dy = 2, 1, 0][BN][8]
+                    const uint64_t ad0 = tc::smem_desc(abase + AX0 * 16, kLboA, 128);
+                    const uint64_t bd0 = tc::smem_desc(bbase, kLboB, 128);
+#pragma unroll 1
+                    for (int h = 0; h < ROWS + 2; ++h)
+                    {
+                        const int dmax = h < 2 ? h : 2;                        // the row taps whose output
+                        const int dmin = h - ROWS + 1 > 0 ? h - ROWS + 1 : 0;  // row h - dy is in the tile
+                        const int nb = dmax - dmin + 1;
+                        const uint32_t id = nb == 3 ? kIdesc3 : (nb == 2 ? kIdesc2 : kIdesc);
+                        const uint32_t dcol = acc + (uint32_t)((h - dmax) * BN);
+                        const bool first = kb == 0 && dmin == 0;  // output row h starts here
+                        const uint64_t adh = tc::desc_at(ad0, (uint32_t)(h * AX * 16));
+                        const uint64_t bdh = tc::desc_at(bd0, (uint32_t)((2 - dmax) * BN * 16));
 #pragma unroll
-                                for (int r = 0; r < ROWS; ++r)
+                        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+                            for (int ks = 0; ks < KC / 16; ++ks)
+                            {
+                                const uint32_t plane = (uint32_t)((dx * (KC / 8) + 2 * ks) * kLboB);
+                                const uint64_t ad = tc::desc_at(adh, (uint32_t)(2 * ks) * kLboA + (uint32_t)(dx * 16));
+                                const uint64_t bd = tc::desc_at(bdh, plane);
+                                if (dx == 0 && ks == 0 && first)
                                 {
-                                    const uint32_t aoff =
-                                        (uint32_t)(2 * ks) * kLboA + (uint32_t)(((r + dy) * AX + dx) * 16);
-                                    const uint64_t ad = tc::smem_desc(abase + aoff, kLboA, 128);
+                                    if (leader)
+                                    {
+                                        tc::mma_bf16(acc + (uint32_t)(h * BN), ad, tc::desc_at(bd0, plane + 2 * BN * 16),
+                                                     kIdesc, 0u);
+                                        if (dmax > 0) tc::mma_bf16(dcol, ad, bd, dmax == 2 ? kIdesc2 : kIdesc, 1u);
+                                    }
+                                }
+                                else if (leader)
+                                    tc::mma_bf16(dcol, ad, bd, id, 1u);
+                            }
+                    }
+                }
+                else
+                {
+                    const uint64_t ad0 = tc::smem_desc(abase, kLboA, 128);
+                    const uint64_t bd0 = tc::smem_desc(bbase, kLboB, 128);
+#pragma unroll 1
+                    for (int tap = 0; tap < 9; ++tap)
+                    {
+                        const int dy = tap / 3, dx = tap % 3;
+                        const uint64_t adt = tc::desc_at(ad0, (uint32_t)((dy * AX + dx) * 16));
+                        const uint64_t bdt = tc::desc_at(bd0, (uint32_t)(tap * (KC / 8) * BN * 16));
+#pragma unroll
+                        for (int ks = 0; ks < KC / 16; ++ks)
+                        {
+                            const uint64_t bd = tc::desc_at(bdt, (uint32_t)(2 * ks * BN * 16));
+#pragma unroll
+                            for (int r = 0; r < ROWS; ++r)
+                            {
+                                const uint64_t ad = tc::desc_at(adt, (uint32_t)(2 * ks) * kLboA + (uint32_t)(r * AX * 16));
+                                if (leader)
                                     tc::mma_bf16(acc + (uint32_t)(r * BN), ad, bd, kIdesc,
                                                  (kb | tap | ks) != 0 ? 1u : 0u);
-                                }
                             }
                         }
                     }
-                    tc::mma_commit(&empty[s]);  // frees the stage when these MMAs retire
                 }
-                if (!ok)
-                {
-                    fail(1);
-                    break;
-                }
-                tc::mma_commit(&acc_full[b]);
+                if (leader) tc::mma_commit(&empty[s]);  // frees the stage when these MMAs retire
             }
-            tc::mma_commit(done);  // completes when every MMA issued above has finished
-            // only the last tiles' epilogues are left: the next layer's blocks may take their places.  (From the
-            // start of the kernel on, they would sit on SMs that other streams' kernels could use: three networks
-            // side by side at 1x256x512 then took 121 us
-            // a pass instead of 111, and one alone 236 instead of 226.)
-            tc::launch_dependents();
+            if (!ok)
+            {
+                if (leader) fail(1);
+                break;
+            }
+            if (leader) tc::mma_commit(&acc_full[b]);
         }
+        if (leader) tc::mma_commit(done);  // completes when every MMA issued above has finished
+        // only the last tiles' epilogues are left: the next layer's blocks may take their places.  (From the
+        // start of the kernel on, they would sit on SMs that other streams' kernels could use: three networks
+        // side by side at 1x256x512 then took 121 us a pass instead of 111, and one alone 236 instead of 226.)
+        tc::launch_dependents();
     }
     else
     {
