@@ -35,8 +35,8 @@
 //
 // What bounds it: 1,050,972 triangles move 244 MB at least (38 us at the copy
 // rate); below 100,000 triangles the chain of dependent launches.  One B200,
-// lg_build_bvh_device with permutation and triangles, wall time: 354 us for
-// 1,050,972 triangles and 124 us for 20,500.  It was 795 and 347 us with a
+// lg_build_bvh_device with permutation and triangles, wall time: 339 us for
+// 1,050,972 triangles and 95 us for 20,500.  It was 795 and 347 us with a
 // second four-pass sort for the BFS order, the refit through L2 at every level
 // and one warp per moved triangle (36 operations).
 #include <algorithm>
@@ -49,6 +49,7 @@
 
 #include "common.h"
 #include "lbvh.cuh"
+#include "pdl.cuh"
 #include "radix_sort.cuh"
 
 namespace lg
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(kTB) bounds_kernel(const lg_triangle* __restri
                                                      unsigned long long* keys, unsigned* ticket,
                                                      float* __restrict__ centroids, float* __restrict__ box)
 {
+    begin_after_predecessors();
     const float third = 1.0f / 3.0f;
     uint64_t mn[3] = {~0ull, ~0ull, ~0ull}, mx[3] = {0, 0, 0};
     for (int t = blockIdx.x * kTB + threadIdx.x; t < n; t += gridDim.x * kTB)
@@ -186,6 +188,7 @@ __global__ void __launch_bounds__(kTB) morton_kernel(const float* __restrict__ c
                                                      const float* __restrict__ box, uint32_t* __restrict__ codes,
                                                      uint32_t* __restrict__ hist)
 {
+    begin_after_predecessors();
     __shared__ uint32_t h[4][256];
     for (int i = threadIdx.x; i < 4 * 256; i += kTB) (&h[0][0])[i] = 0;
     __syncthreads();
@@ -233,6 +236,7 @@ __global__ void __launch_bounds__(kChunk) tree_kernel(const uint32_t* __restrict
                                                       int* __restrict__ gap_l, int* __restrict__ gap_r,
                                                       int* __restrict__ gap_parent, int2* __restrict__ skip)
 {
+    begin_after_predecessors();
     constexpr int kNear = 4;
     __shared__ uint32_t s_code[kChunk + 2];  // codes base - 1 .. base + kChunk
     __shared__ int s_l[kChunk], s_r[kChunk], s_list[2 * kChunk], s_listed;
@@ -375,6 +379,7 @@ __global__ void __launch_bounds__(kChunk) depth_kernel(int n, const int* __restr
                                                        const int2* __restrict__ skip, uchar2* __restrict__ depth,
                                                        int* __restrict__ counts, int chunks)
 {
+    begin_after_predecessors();
     __shared__ int h[kMaxDepths];
     if (threadIdx.x < kMaxDepths) h[threadIdx.x] = 0;
     __syncthreads();
@@ -412,6 +417,7 @@ __global__ void __launch_bounds__(kChunk) depth_kernel(int n, const int* __restr
 // Exclusive scan of each depth's row of counts, one block per depth, and the row totals.
 __global__ void __launch_bounds__(kTB) depth_scan_kernel(int* __restrict__ counts, int chunks, int* __restrict__ totals)
 {
+    begin_after_predecessors();
     __shared__ int warp_sums[kTB / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int* row = counts + (size_t)blockIdx.x * chunks;
@@ -464,6 +470,7 @@ __global__ void __launch_bounds__(kChunk) bfs_kernel(int n, const uchar2* __rest
                                                      const int* __restrict__ totals, int* __restrict__ bfs_gap,
                                                      int* __restrict__ bfs_leaf, int* __restrict__ n_nodes)
 {
+    begin_after_predecessors();
     constexpr int kWarps = kChunk / 32;
     __shared__ unsigned masks[kWarps][2][kMaxDepths];  // lanes whose gap / leaf has this depth
     __shared__ int first[kWarps][kMaxDepths];          // index of the warp's first node of the depth
@@ -614,6 +621,7 @@ __global__ void __launch_bounds__(kChunk)
                 int32_t* __restrict__ perm_out, lg_bvh_node* nodes, TopNode* __restrict__ tops,
                 int* __restrict__ n_tops)
 {
+    begin_after_predecessors();
     extern __shared__ __align__(16) unsigned char emit_mem[];
     EmitShared& sh = *reinterpret_cast<EmitShared*>(emit_mem);
     const int base = blockIdx.x * kChunk, t = threadIdx.x, k = base + t;
@@ -764,6 +772,7 @@ __global__ void __launch_bounds__(kTopThreads)
                const int* __restrict__ bfs_gap, TopNode* __restrict__ tops_out, int* __restrict__ n_tops_out,
                lg_bvh_node* nodes)
 {
+    begin_after_predecessors();
     extern __shared__ __align__(16) unsigned char emit_mem[];
     TopShared& sh = *reinterpret_cast<TopShared*>(emit_mem);
     const int first = blockIdx.x * kGroup, have = min(kGroup, groups_in - first);
@@ -953,27 +962,29 @@ int lbvh_build(const lg_triangle* d_tris, int n, lg_bvh_node* d_nodes, int* n_no
     LG_TRY_CUDA(cudaMemsetAsync(rs.hist, 0, rs.zero_bytes, stream));
     rs.error = (uint32_t*)(result + 1);
     const int grid = std::min(blocks_for((size_t)n), 148 * 8);
-    bounds_kernel<<<grid, kTB, 0, stream>>>(d_tris, n, keys, ticket, centroids, box);
-    morton_kernel<<<std::min(grid, 148 * 4), kTB, 0, stream>>>(centroids, n, box, codes, rs.hist);
+    LG_TRY_CUDA(launch_dependent(bounds_kernel, grid, kTB, 0, stream, d_tris, n, keys, ticket, centroids, box));
+    LG_TRY_CUDA(launch_dependent(morton_kernel, std::min(grid, 148 * 4), kTB, 0, stream, centroids, n, box, codes,
+                                 rs.hist));
     // 30-bit codes, stable: ties stay in input order
     LG_TRY_CUDA(radix_sort_pairs(codes, idx, (size_t)n, 0, 30, rs, stream, true, true));
-    tree_kernel<<<chunks, kChunk, 0, stream>>>(codes, n, gl, gr, gp, skip);
-    depth_kernel<<<chunks, kChunk, 0, stream>>>(n, gp, skip, depth, counts, chunks);
-    depth_scan_kernel<<<kMaxDepths, kTB, 0, stream>>>(counts, chunks, totals);
-    bfs_kernel<<<chunks, kChunk, 0, stream>>>(n, depth, counts, chunks, totals, bfs_gap, bfs_leaf, result);
+    LG_TRY_CUDA(launch_dependent(tree_kernel, chunks, kChunk, 0, stream, codes, n, gl, gr, gp, skip));
+    LG_TRY_CUDA(launch_dependent(depth_kernel, chunks, kChunk, 0, stream, n, gp, skip, depth, counts, chunks));
+    LG_TRY_CUDA(launch_dependent(depth_scan_kernel, kMaxDepths, kTB, 0, stream, counts, chunks, totals));
+    LG_TRY_CUDA(launch_dependent(bfs_kernel, chunks, kChunk, 0, stream, n, depth, counts, chunks, totals, bfs_gap,
+                                 bfs_leaf, result));
     lg_triangle* tris_sorted = need_tmp ? (lg_triangle*)at(L.off_tmp_tris) : d_tris_out;
     LG_TRY_CUDA(cudaFuncSetAttribute((const void*)emit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(EmitShared)));
-    emit_kernel<<<chunks, kChunk, sizeof(EmitShared), stream>>>(d_tris, idx, n, gl, gr, gp, bfs_gap, bfs_leaf,
-                                                                      tris_sorted, d_perm_out, d_nodes, tops, n_tops);
+    LG_TRY_CUDA(launch_dependent(emit_kernel, chunks, kChunk, (int)sizeof(EmitShared), stream, d_tris, idx, n, gl,
+                                 gr, gp, bfs_gap, bfs_leaf, tris_sorted, d_perm_out, d_nodes, tops, n_tops));
     LG_TRY_CUDA(cudaFuncSetAttribute((const void*)top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(TopShared)));
     long long span = kChunk;
     for (int groups = chunks; groups > 1;)
     {
         const int out = (groups + kGroup - 1) / kGroup;
-        top_kernel<<<out, kTopThreads, sizeof(TopShared), stream>>>(tops, n_tops, groups, span, n, gl, gr, gp, bfs_gap,
-                                                                     tops2, n_tops2, d_nodes);
+        LG_TRY_CUDA(launch_dependent(top_kernel, out, kTopThreads, (int)sizeof(TopShared), stream, tops, n_tops,
+                                     groups, span, n, gl, gr, gp, bfs_gap, tops2, n_tops2, d_nodes));
         std::swap(tops, tops2);
         std::swap(n_tops, n_tops2);
         groups = out;

@@ -2,11 +2,13 @@
 //
 // Bound by latency at the sizes the library sorts (8 MB of pairs stay in L2): a
 // pass is one round of key loads, the ranking, the look-back and the writes.
-// One B200, 30-bit keys (4 passes): 59 us for 1,050,972 pairs and 21 us for
+// One B200, 30-bit keys (4 passes, launched one after the other): 59 us for 1,050,972 pairs and 21 us for
 // 20,500.  With three launches a pass (per-tile histogram, scan of the
 // [digit][tile] table, scatter with a block-wide sync per 256 keys) a pass took 30
 // and 20 us.
 #include "radix_sort.cuh"
+
+#include "pdl.cuh"
 
 namespace lg
 {
@@ -28,6 +30,7 @@ __global__ void __launch_bounds__(kHistThreads) hist_kernel(const uint32_t* __re
 {
     __shared__ uint32_t h[kRadixMaxPasses][256];
     for (int i = threadIdx.x; i < kRadixMaxPasses * 256; i += kHistThreads) (&h[0][0])[i] = 0;
+    begin_after_predecessors();
     __syncthreads();
     for (size_t i = (size_t)blockIdx.x * kHistThreads + threadIdx.x; i < n; i += (size_t)gridDim.x * kHistThreads)
     {
@@ -97,8 +100,9 @@ __global__ void __launch_bounds__(kThreads) pass_kernel(const uint32_t* __restri
     extern __shared__ __align__(16) unsigned char pass_mem[];
     PassShared<kThreads, kItems>& sh = *reinterpret_cast<PassShared<kThreads, kItems>*>(pass_mem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) sh.tile = atomicAdd(ticket, 1u);
     for (int i = tid; i < kWarps * 256; i += kThreads) (&sh.warp_cnt[0][0])[i] = 0;
+    begin_after_predecessors();
+    if (tid == 0) sh.tile = atomicAdd(ticket, 1u);
     const uint32_t digit_total = tid < 256 ? hist[tid] : 0u;
     __syncthreads();
     const uint32_t tile = sh.tile;
@@ -221,9 +225,8 @@ cudaError_t launch_pass(const PassArgs& a, bool iota, size_t tiles, cudaStream_t
     auto k = iota ? pass_kernel<kThreads, kItems, true> : pass_kernel<kThreads, kItems, false>;
     const cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    k<<<(unsigned)tiles, kThreads, smem, st>>>(a.ki, a.vi, a.ko, a.vo, a.n, a.shift, a.bits, a.hist, a.state, a.ticket,
-                                               a.error);
-    return cudaGetLastError();
+    return launch_dependent(k, (unsigned)tiles, kThreads, smem, st, a.ki, a.vi, a.ko, a.vo, a.n, a.shift, a.bits, a.hist,
+                            a.state, a.ticket, a.error);
 }
 }  // namespace
 
@@ -267,9 +270,9 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, size_t n, int begin
     if (!counted)
     {
         const size_t blocks = (n + kHistThreads * 4 - 1) / (kHistThreads * 4);
-        hist_kernel<<<(unsigned)(blocks < 592 ? blocks : 592), kHistThreads, 0, stream>>>(keys, n, begin_bit, end_bit,
-                                                                                        s.hist);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        e = launch_dependent(hist_kernel, (unsigned)(blocks < 592 ? blocks : 592), kHistThreads, 0, stream, keys, n,
+                             begin_bit, end_bit, s.hist);
+        if (e != cudaSuccess) return e;
     }
     uint32_t *ki = keys, *vi = vals, *ko = s.keys_alt, *vo = s.vals_alt;
     int pass = 0;

@@ -30,6 +30,7 @@
 
 #include "bvh.h"
 #include "common.h"
+#include "pdl.cuh"
 #include "radix_sort.cuh"
 #include "render_tree.cuh"
 
@@ -67,6 +68,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int* warp_sums, int& total
 }
 __global__ void scan_local_kernel(const int* __restrict__ in, int n, int* __restrict__ out, int* __restrict__ sums)
 {
+    begin_after_predecessors();
     __shared__ int ws[kTB / 32];
     const int i = blockIdx.x * kTB + threadIdx.x;
     int total;
@@ -76,6 +78,7 @@ __global__ void scan_local_kernel(const int* __restrict__ in, int n, int* __rest
 }
 __global__ void scan_sums_kernel(int* __restrict__ sums, int nb, int* __restrict__ grand_total)
 {
+    begin_after_predecessors();
     __shared__ int ws[kTB / 32];
     __shared__ int carry;
     if (threadIdx.x == 0) carry = 0;
@@ -94,6 +97,7 @@ __global__ void scan_sums_kernel(int* __restrict__ sums, int nb, int* __restrict
 }
 __global__ void scan_add_kernel(int* __restrict__ out, int n, const int* __restrict__ sums)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * kTB + threadIdx.x;
     if (i < n) out[i] += sums[blockIdx.x];
 }
@@ -102,14 +106,15 @@ cudaError_t excl_scan(const int* in, int n, int* out, int* sums, int* total, cud
 {
     const int nb = (n + kTB - 1) / kTB;
     if (n <= 0) return cudaMemsetAsync(total, 0, sizeof(int), st);
-    scan_local_kernel<<<nb, kTB, 0, st>>>(in, n, out, sums);
-    scan_sums_kernel<<<1, kTB, 0, st>>>(sums, nb, total);
-    scan_add_kernel<<<nb, kTB, 0, st>>>(out, n, sums);
-    return cudaGetLastError();
+    cudaError_t e = launch_dependent(scan_local_kernel, nb, kTB, 0, st, in, n, out, sums);
+    if (e == cudaSuccess) e = launch_dependent(scan_sums_kernel, 1, kTB, 0, st, sums, nb, total);
+    if (e == cudaSuccess) e = launch_dependent(scan_add_kernel, nb, kTB, 0, st, out, n, sums);
+    return e;
 }
 // ---- depth order ----
 __global__ void parent_of_kernel(const lg_bvh_node* __restrict__ nodes, int n, int* __restrict__ parent)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * kTB + threadIdx.x;
     if (i >= n) return;
     const lg_bvh_node nd = nodes[i];
@@ -122,6 +127,7 @@ __global__ void parent_of_kernel(const lg_bvh_node* __restrict__ nodes, int n, i
 __global__ void depth_of_kernel(int n, int root, const int* __restrict__ parent, uint32_t* __restrict__ depth,
                                 uint32_t* __restrict__ ids)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * kTB + threadIdx.x;
     if (i >= n) return;
     uint32_t d = 0;
@@ -132,6 +138,7 @@ __global__ void depth_of_kernel(int n, int root, const int* __restrict__ parent,
 }
 __global__ void rank_kernel(const uint32_t* __restrict__ order, int n, int* __restrict__ newpos)
 {
+    begin_after_predecessors();
     const int r = blockIdx.x * kTB + threadIdx.x;
     if (r < n) newpos[order[r]] = r;
 }
@@ -142,6 +149,7 @@ constexpr int kEmitNodes = 256;
 __global__ void __launch_bounds__(kTB) emit_kernel(const lg_bvh_node* __restrict__ in, const uint32_t* __restrict__ order,
                                                    const int* __restrict__ newpos, int n, lg_bvh_node* __restrict__ out)
 {
+    begin_after_predecessors();
     __shared__ uint32_t s_src[kEmitNodes];
     const int base = blockIdx.x * kEmitNodes, cnt = min(kEmitNodes, n - base);
     for (int i = threadIdx.x; i < cnt; i += kTB) s_src[i] = order[base + i];
@@ -161,6 +169,7 @@ __global__ void __launch_bounds__(kTB) emit_kernel(const lg_bvh_node* __restrict
 // Where each depth's nodes begin in depth order, from the sort's counts of the 256 depths; start[256] = n.
 __global__ void level_start_kernel(const uint32_t* __restrict__ counts, int n, int* __restrict__ start)
 {
+    begin_after_predecessors();
     __shared__ int ws[kTB / 32];
     int total;
     const int e = block_excl_scan((int)counts[threadIdx.x], ws, total);
@@ -190,6 +199,7 @@ __device__ __forceinline__ Box join(const Box& a, const Box& b)
 __global__ void leaf_at_kernel(const lg_bvh_node* __restrict__ nodes, int n, int* __restrict__ leaf_at,
                                int* __restrict__ flag)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * kTB + threadIdx.x;
     if (i >= n) return;
     const lg_bvh_node nd = nodes[i];
@@ -204,6 +214,7 @@ __global__ void init_clusters_kernel(const lg_bvh_node* __restrict__ nodes, cons
                                      const int* __restrict__ flag, const int* __restrict__ pos, int n_tris,
                                      lg_bvh_node* __restrict__ tn, int* __restrict__ cid, Box* __restrict__ cbox)
 {
+    begin_after_predecessors();
     const int t = blockIdx.x * kTB + threadIdx.x;
     if (t >= n_tris || !flag[t]) return;
     const int k = pos[t];
@@ -219,6 +230,7 @@ __global__ void init_clusters_kernel(const lg_bvh_node* __restrict__ nodes, cons
 __global__ void init_tri_clusters_kernel(const lg_triangle* __restrict__ tris, int n_tris,
                                          lg_bvh_node* __restrict__ tn, int* __restrict__ cid, Box* __restrict__ cbox)
 {
+    begin_after_predecessors();
     const int t = blockIdx.x * kTB + threadIdx.x;
     if (t >= n_tris) return;
     const lg_triangle tr = tris[t];
@@ -245,6 +257,7 @@ __global__ void init_tri_clusters_kernel(const lg_triangle* __restrict__ tris, i
 __global__ void __launch_bounds__(kTB) nn_kernel(const Box* __restrict__ cbox, const int* __restrict__ dc,
                                                  int* __restrict__ nn)
 {
+    begin_after_predecessors();
     __shared__ Box sb[kTB + 2 * kRadius];
     const int c = *dc;
     const int base = blockIdx.x * kTB - kRadius;
@@ -283,6 +296,7 @@ __global__ void round_flags_kernel(const int* __restrict__ nn, const int* __rest
                                    int* __restrict__ kflag, int* __restrict__ midx, int* __restrict__ kpos,
                                    int* __restrict__ msums, int* __restrict__ ksums)
 {
+    begin_after_predecessors();
     __shared__ int ws[kTB / 32];
     const int c = cur[0];
     const int i = blockIdx.x * kTB + threadIdx.x;
@@ -314,6 +328,7 @@ constexpr int kSumThreads = 1024;
 __global__ void __launch_bounds__(kSumThreads) round_sums_kernel(int* __restrict__ msums, int* __restrict__ ksums, int nb,
                                                                  const int* __restrict__ cur, int* __restrict__ nxt)
 {
+    begin_after_predecessors();
     __shared__ int ws[2][kSumThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int per = (nb + kSumThreads - 1) / kSumThreads;  // consecutive entries per thread
@@ -374,6 +389,7 @@ __global__ void round_apply_kernel(const int* __restrict__ nn, const int* __rest
                                    Box* __restrict__ cbox, lg_bvh_node* __restrict__ tn, int* __restrict__ cid2,
                                    Box* __restrict__ cbox2)
 {
+    begin_after_predecessors();
     const int c = cur[0], node_base = cur[1];
     const int i = blockIdx.x * kTB + threadIdx.x;
     if (i >= c) return;
@@ -421,6 +437,7 @@ __global__ void __launch_bounds__(kTailThreads) rounds_tail_kernel(const int* __
                                                                    int* __restrict__ state, lg_bvh_node* __restrict__ tn,
                                                                    int* __restrict__ root)
 {
+    begin_after_predecessors();
     extern __shared__ __align__(16) unsigned char tail_mem[];
     TailShared& sh = *reinterpret_cast<TailShared*>(tail_mem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -640,16 +657,19 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
         int c = 0;
         if (mode == 2)
         {
-            init_tri_clusters_kernel<<<(t + kTB - 1) / kTB, kTB, 0, st>>>(d_tris, t, tn, cid, cbox);
+            LG_TRY_CUDA(launch_dependent(init_tri_clusters_kernel, (t + kTB - 1) / kTB, kTB, 0, st, d_tris, t, tn,
+                                         cid, cbox));
             LG_TRY_CUDA(cudaGetLastError());
             c = t;
         }
         else
         {
             LG_TRY_CUDA(cudaMemsetAsync(flag, 0, sizeof(int) * (size_t)t, st));
-            leaf_at_kernel<<<(in_nodes + kTB - 1) / kTB, kTB, 0, st>>>(d_nodes, in_nodes, leaf_at, flag);
+            LG_TRY_CUDA(launch_dependent(leaf_at_kernel, (in_nodes + kTB - 1) / kTB, kTB, 0, st, d_nodes, in_nodes,
+                                         leaf_at, flag));
             LG_TRY_CUDA(excl_scan(flag, t, pos, sums, totals, st));
-            init_clusters_kernel<<<(t + kTB - 1) / kTB, kTB, 0, st>>>(d_nodes, leaf_at, flag, pos, t, tn, cid, cbox);
+            LG_TRY_CUDA(launch_dependent(init_clusters_kernel, (t + kTB - 1) / kTB, kTB, 0, st, d_nodes, leaf_at,
+                                         flag, pos, t, tn, cid, cbox));
             LG_TRY_CUDA(cudaGetLastError());
             LG_TRY_CUDA(cudaMemcpyAsync(&c, totals, sizeof(int), cudaMemcpyDeviceToHost, st));
             LG_TRY_CUDA(cudaStreamSynchronize(st));
@@ -670,11 +690,12 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
             {
                 const int* sc = sbuf[cur];
                 int* sn = sbuf[cur ^ 1];
-                nn_kernel<<<gc, kTB, 0, st>>>(cbox, sc, nn);
-                round_flags_kernel<<<gc, kTB, 0, st>>>(nn, sc, mflag, kflag, midx, kpos, sums, ksums);
-                round_sums_kernel<<<1, kSumThreads, 0, st>>>(sums, ksums, gc, sc, sn);
-                round_apply_kernel<<<gc, kTB, 0, st>>>(nn, sc, mflag, kflag, midx, kpos, sums, ksums, cid, cbox, tn,
-                                                       cid2, cbox2);
+                LG_TRY_CUDA(launch_dependent(nn_kernel, gc, kTB, 0, st, cbox, sc, nn));
+                LG_TRY_CUDA(launch_dependent(round_flags_kernel, gc, kTB, 0, st, nn, sc, mflag, kflag, midx, kpos,
+                                             sums, ksums));
+                LG_TRY_CUDA(launch_dependent(round_sums_kernel, 1, kSumThreads, 0, st, sums, ksums, gc, sc, sn));
+                LG_TRY_CUDA(launch_dependent(round_apply_kernel, gc, kTB, 0, st, nn, sc, mflag, kflag, midx, kpos,
+                                             sums, ksums, cid, cbox, tn, cid2, cbox2));
                 LG_TRY_CUDA(cudaGetLastError());
                 int* ti = cid; cid = cid2; cid2 = ti;
                 Box* tb = cbox; cbox = cbox2; cbox2 = tb;
@@ -687,7 +708,8 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
         int* droot = totals + 24;
         LG_TRY_CUDA(cudaFuncSetAttribute((const void*)rounds_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)sizeof(TailShared)));
-        rounds_tail_kernel<<<1, kTailThreads, sizeof(TailShared), st>>>(cid, cbox, sbuf[cur], tn, droot);
+        LG_TRY_CUDA(launch_dependent(rounds_tail_kernel, 1, kTailThreads, (int)sizeof(TailShared), st, cid, cbox,
+                                     sbuf[cur], tn, droot));
         LG_TRY_CUDA(cudaGetLastError());
         LG_TRY_CUDA(cudaMemcpyAsync(hstate, sbuf[cur], sizeof(hstate), cudaMemcpyDeviceToHost, st));
         LG_TRY_CUDA(cudaMemcpyAsync(&root, droot, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -699,17 +721,18 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
     }
     // Depth order: a stable sort of node ids by depth (ids ascending within a depth).
     LG_TRY_CUDA(cudaMemsetAsync(parent, 0xff, sizeof(int) * (size_t)n_nodes, st));
-    parent_of_kernel<<<g, kTB, 0, st>>>(src, n_nodes, parent);
-    depth_of_kernel<<<g, kTB, 0, st>>>(n_nodes, root, parent, depth, ids);
+    LG_TRY_CUDA(launch_dependent(parent_of_kernel, g, kTB, 0, st, src, n_nodes, parent));
+    LG_TRY_CUDA(launch_dependent(depth_of_kernel, g, kTB, 0, st, n_nodes, root, parent, depth, ids));
     LG_TRY_CUDA(cudaGetLastError());
     const RadixSortScratch rs = radix_sort_bind(sort_mem, (size_t)n_nodes);
     LG_TRY_CUDA(radix_sort_pairs(depth, ids, (size_t)n_nodes, 0, 8, rs, st));
     uint32_t max_depth = 0, sort_error = 0;
     LG_TRY_CUDA(cudaMemcpyAsync(&sort_error, rs.error, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     LG_TRY_CUDA(cudaMemcpyAsync(&max_depth, depth + n_nodes - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    rank_kernel<<<g, kTB, 0, st>>>(ids, n_nodes, newpos);
-    emit_kernel<<<(n_nodes + kEmitNodes - 1) / kEmitNodes, kTB, 0, st>>>(src, ids, newpos, n_nodes, d_out);
-    level_start_kernel<<<1, kTB, 0, st>>>(rs.hist, n_nodes, d_level_start);
+    LG_TRY_CUDA(launch_dependent(rank_kernel, g, kTB, 0, st, ids, n_nodes, newpos));
+    LG_TRY_CUDA(launch_dependent(emit_kernel, (n_nodes + kEmitNodes - 1) / kEmitNodes, kTB, 0, st, src, ids, newpos,
+                                 n_nodes, d_out));
+    LG_TRY_CUDA(launch_dependent(level_start_kernel, 1, kTB, 0, st, rs.hist, n_nodes, d_level_start));
     LG_TRY_CUDA(cudaMemcpyAsync(level_start_host, d_level_start, 257 * sizeof(int), cudaMemcpyDeviceToHost, st));
     LG_TRY_CUDA(cudaGetLastError());
     LG_TRY_CUDA(cudaStreamSynchronize(st));

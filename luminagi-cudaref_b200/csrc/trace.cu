@@ -39,6 +39,7 @@
 #include <cuda_runtime.h>
 
 #include "trace.cuh"
+#include "pdl.cuh"
 
 namespace lg
 {
@@ -56,6 +57,7 @@ constexpr int kScanTB = 1024;
 
 __global__ void flags_kernel(const lg_bvh_node* __restrict__ nodes, int n, int* __restrict__ is_internal)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) is_internal[i] = nodes[i].triCount == 0 ? 1 : 0;
 }
@@ -97,6 +99,7 @@ __device__ int block_exclusive_scan(int v, int* total)
 __global__ void __launch_bounds__(kScanTB) count_kernel(const int* __restrict__ is_internal, int n,
                                                         int* __restrict__ block_sums)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * kScanTB + threadIdx.x;
     int v = i < n ? is_internal[i] : 0;
     int total;
@@ -106,6 +109,7 @@ __global__ void __launch_bounds__(kScanTB) count_kernel(const int* __restrict__ 
 // Pass 2: scan of block sums (single block, loops).
 __global__ void __launch_bounds__(kScanTB) scan_sums_kernel(int* __restrict__ block_sums, int nb)
 {
+    begin_after_predecessors();
     __shared__ int carry;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -125,6 +129,7 @@ __global__ void __launch_bounds__(kScanTB) scan_sums_kernel(int* __restrict__ bl
 __global__ void __launch_bounds__(kScanTB) dense_kernel(const int* __restrict__ is_internal, int n,
                                                         const int* __restrict__ block_sums, int* __restrict__ dense)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * kScanTB + threadIdx.x;
     int v = i < n ? is_internal[i] : 0;
     int total;
@@ -140,6 +145,7 @@ __device__ __forceinline__ int child_link(const lg_bvh_node* nodes, const int* d
 __global__ void wide_kernel(const lg_bvh_node* __restrict__ nodes, int n, const int* __restrict__ dense,
                             WideNode* __restrict__ wide, int2* __restrict__ leaves)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const lg_bvh_node nd = nodes[i];
@@ -195,6 +201,7 @@ __global__ void __launch_bounds__(kSelectThreads) select4_kernel(const lg_bvh_no
                                                                  int* __restrict__ is4, int* __restrict__ sel,
                                                                  int* __restrict__ rb, int* __restrict__ bound)
 {
+    begin_after_predecessors();
     const int i = lo + blockIdx.x * kSelectThreads + threadIdx.x;
     int here = 0;
     if (i < hi)
@@ -305,6 +312,7 @@ __global__ void wide4_kernel(const lg_bvh_node* __restrict__ nodes, int n, const
                              const int* __restrict__ dense4, const int* __restrict__ dense2,
                              const int* __restrict__ sel, Wide4Node* __restrict__ out, int inline_ok, int null_link)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || !is4[i]) return;
     float lo[3][4], hi[3][4];
@@ -328,6 +336,7 @@ __global__ void wide4_kernel(const lg_bvh_node* __restrict__ nodes, int n, const
 
 __global__ void tri_prep_kernel(const lg_triangle* __restrict__ tris, int n, float4* __restrict__ tv, int watertight)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const lg_triangle t = tris[i];
@@ -715,12 +724,15 @@ cudaError_t build_wide_nodes(const lg_bvh_node* d_nodes, int n_nodes, WideNode* 
     int* is_internal = d_scratch;
     int* dense = d_scratch + n_nodes;
     int* block_sums = d_scratch + 2 * (size_t)n_nodes;
-    flags_kernel<<<nb, kScanTB, 0, stream>>>(d_nodes, n_nodes, is_internal);
-    count_kernel<<<nb, kScanTB, 0, stream>>>(is_internal, n_nodes, block_sums);
-    scan_sums_kernel<<<1, kScanTB, 0, stream>>>(block_sums, nb);
-    dense_kernel<<<nb, kScanTB, 0, stream>>>(is_internal, n_nodes, block_sums, dense);
-    wide_kernel<<<(n_nodes + 255) / 256, 256, 0, stream>>>(d_nodes, n_nodes, dense, d_wide, d_leaves);
-    return cudaGetLastError();
+    cudaError_t e = launch_dependent(flags_kernel, nb, kScanTB, 0, stream, d_nodes, n_nodes, is_internal);
+    if (e == cudaSuccess) e = launch_dependent(count_kernel, nb, kScanTB, 0, stream, is_internal, n_nodes,
+                                               block_sums);
+    if (e == cudaSuccess) e = launch_dependent(scan_sums_kernel, 1, kScanTB, 0, stream, block_sums, nb);
+    if (e == cudaSuccess) e = launch_dependent(dense_kernel, nb, kScanTB, 0, stream, is_internal, n_nodes,
+                                               block_sums, dense);
+    if (e == cudaSuccess) e = launch_dependent(wide_kernel, (n_nodes + 255) / 256, 256, 0, stream, d_nodes, n_nodes,
+                                               dense, d_wide, d_leaves);
+    return e;
 }
 
 cudaError_t build_wide4_nodes(const lg_bvh_node* d_nodes, int n_nodes, int n_tris, int null_leaf,
@@ -750,17 +762,19 @@ cudaError_t build_wide4_nodes(const lg_bvh_node* d_nodes, int n_nodes, int n_tri
     {
         const int lo = level_start[d], hi = level_start[d + 1];
         if (hi > lo)
-            select4_kernel<<<(hi - lo + kSelectThreads - 1) / kSelectThreads, kSelectThreads, 0, stream>>>(
-                d_nodes, lo, hi, is4, sel, rb, bound);
+            if (e == cudaSuccess) e = launch_dependent(select4_kernel,
+                                                       (hi - lo + kSelectThreads - 1) / kSelectThreads,
+                                                       kSelectThreads, 0, stream, d_nodes, lo, hi, is4, sel, rb,
+                                                       bound);
     }
-    count_kernel<<<nb, kScanTB, 0, stream>>>(is4, n_nodes, sums4);
-    scan_sums_kernel<<<1, kScanTB, 0, stream>>>(sums4, nb);
-    dense_kernel<<<nb, kScanTB, 0, stream>>>(is4, n_nodes, sums4, dense4);
+    if (e == cudaSuccess) e = launch_dependent(count_kernel, nb, kScanTB, 0, stream, is4, n_nodes, sums4);
+    if (e == cudaSuccess) e = launch_dependent(scan_sums_kernel, 1, kScanTB, 0, stream, sums4, nb);
+    if (e == cudaSuccess) e = launch_dependent(dense_kernel, nb, kScanTB, 0, stream, is4, n_nodes, sums4, dense4);
     const int inline_ok = n_tris < (1 << 27) ? 1 : 0;
     *leaf_inline_host = inline_ok;
     const int null_link = inline_ok ? ~(null_leaf << 4) : ~null_leaf;
-    wide4_kernel<<<g, tb, 0, stream>>>(d_nodes, n_nodes, is4, dense4, dense2, sel, d_wide4, inline_ok, null_link);
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_dependent(wide4_kernel, g, tb, 0, stream, d_nodes, n_nodes, is4, dense4, dense2,
+                                               sel, d_wide4, inline_ok, null_link);
     if (e != cudaSuccess) return e;
     int last_d = 0, last_v = 0, stack4 = 0, root_internal = 0;
     e = cudaMemcpyAsync(&last_d, dense4 + n_nodes - 1, sizeof(int), cudaMemcpyDeviceToHost, stream);
@@ -781,8 +795,8 @@ cudaError_t build_wide4_nodes(const lg_bvh_node* d_nodes, int n_nodes, int n_tri
 cudaError_t prepare_triangles(const lg_triangle* d_tris, int n, float4* d_tv, bool watertight, cudaStream_t stream)
 {
     if (n <= 0) return cudaSuccess;
-    tri_prep_kernel<<<(n + 255) / 256, 256, 0, stream>>>(d_tris, n, d_tv, watertight ? 1 : 0);
-    return cudaGetLastError();
+    return launch_dependent(tri_prep_kernel, (n + 255) / 256, 256, 0, stream, d_tris, n, d_tv,
+                            watertight ? 1 : 0);
 }
 
 template <bool kCount, bool kAcc64, int W, bool kWT, bool kBatch = false, bool kTop = false, bool kChecked = true>

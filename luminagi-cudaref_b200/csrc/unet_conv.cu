@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include "common.h"
+#include "pdl.cuh"
 #include "tc_ptx.cuh"
 #include "unet_conv.cuh"
 
@@ -990,24 +991,6 @@ cudaError_t make_map_chunked(CUtensorMap* m, const __nv_bfloat16* base, int N, i
 // Dynamic shared memory a CTA may use on sm_100: 227 KB less 2 KB of headroom
 // for the kernel's static shared memory (the epilogue constants, 1.4 KB).
 constexpr int kMaxSmem = 225 * 1024;
-
-// A launch whose blocks may start while the previous kernel of the stream is still running; every kernel
-// launched so waits (wait_for_predecessors) before it touches device memory.
-template <class... P, class... A>
-cudaError_t launch_dependent(void (*fn)(P...), dim3 grid, int block, int smem, cudaStream_t stream, A&&... args)
-{
-    cudaLaunchConfig_t c{};
-    c.gridDim = grid;
-    c.blockDim = dim3((unsigned)block);
-    c.dynamicSmemBytes = (size_t)smem;
-    c.stream = stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, fn, std::forward<A>(args)...);
-}
 
 template <int BN, int KC, int STAGES, int EPI, bool RESW = false, int ROWS = kRows, bool DYP = false, bool VUP = false>
 cudaError_t launch_persistent(const __nv_bfloat16* in, const ConvArgs& a, cudaStream_t stream, ConvPlan& plan)
