@@ -759,7 +759,8 @@ __global__ void __launch_bounds__(pthreads(EPI), 1) conv3x3_tc_persistent(const 
         // and a descriptor is the stage's own plus an offset instead of built anew for each MMA.  Both together,
         // against lane 0 alone building each one: 622 -> 611 us a pass at 1x864x1728, 550 -> 541 (HDR, 1x720x1280),
         // 4.71 -> 4.66 ms at 8x864x1728, 157.2 -> 155.5 us at 1x128x128, 178.6 -> 178.6 at 1x256x512 with 12
-        // channels.  What each of the two gives was not measured apart.
+        // channels.  With the offsets but lane 0 alone in the loops: 4.43 ms against 4.38 at 8x864x1728, 157.6 us
+        // against 155.4 at 1x128x128.
         const bool leader = lane == 0;
         int it = 0, j = 0;
         if (RESW && !tc::mbar_wait(wfull, 0) && leader) fail(5);
