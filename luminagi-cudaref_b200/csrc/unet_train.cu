@@ -290,7 +290,7 @@ int loss_and_grads(lg_unet* u, const float* d_x, const float* d_t, int N, int H,
         a.Cin_real = layer_cin_real(u, L);
         a.dw = G + u->w_off[L];
         a.err = (int*)u->err.p;
-        LG_TRY(u->wpart.ensure(conv3x3_wgrad_partial_floats(N, a.H, a.Cout, a.Cin, a.Cin_real, u->sm_count) *
+        LG_TRY(u->wpart.ensure(conv3x3_wgrad_partial_floats(N, a.H, a.W, a.Cout, a.Cin, a.Cin_real, u->sm_count) *
                                sizeof(float)));
         a.partial = (float*)u->wpart.p;
         LG_TRY_CUDA(conv3x3_wgrad((const bf*)u->dz[L].p, (const bf*)in_of[L], a, u->sm_count, side));

@@ -21,7 +21,7 @@ struct WgradArgs
 };
 
 // Floats of WgradArgs::partial the launch for this layer shape needs.
-size_t conv3x3_wgrad_partial_floats(int N, int H, int Cout, int Cin, int Cin_real, int sm_count);
+size_t conv3x3_wgrad_partial_floats(int N, int H, int W, int Cout, int Cin, int Cin_real, int sm_count);
 // dW += sum over pixels of dZ (x) shifted X; both blocked BF16 at N x C x H x W.
 cudaError_t conv3x3_wgrad(const __nv_bfloat16* dz, const __nv_bfloat16* x, const WgradArgs& a, int sm_count,
                           cudaStream_t stream);
