@@ -68,10 +68,11 @@ struct WSmem
     }
 };
 
-// The MMAs of one K-step of rows of 16 * NK pixels.  One thread issues them and sets the kernel's pace, so the
-// row shape is a constant and each descriptor the stage's own plus an offset: with descriptors built one by
-// one in loops a training pass of 16x128x128 took 1.49 ms, with this 1.32.  (All lanes of a warp
-// walking the loops and one issuing: 1.50.)
+// The MMAs of one K-step of rows of 16 * NK pixels, all issued by one thread.  The row shape is a constant and
+// each descriptor the stage's own plus an offset: a training pass of 16x128x128 took 1.50 ms with descriptors
+// built one by one in loops, 1.41 with this.  Two other forms, measured against 1.32 for this one with a
+// faster tail pass: the row shape at run time 1.40, and all lanes of a warp walking those loops with one
+// issuing 1.50.
 template <int NK, int BNW>
 __device__ __forceinline__ void step_mmas(uint32_t tmem, uint64_t ad0, uint64_t bd0, uint32_t idesc, bool accumulate)
 {
