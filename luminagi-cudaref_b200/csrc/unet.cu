@@ -260,13 +260,18 @@ int lg_unet_create(int base, int in_ch, int act_mode, lg_unet** out)
     u->in_ch = in_ch;
     u->n_params = layout_params(u);
     // Forward tiles: lg_unet_autotune's choice at batch 8, 1728x864 on B200 (7.05 ms, against 8.92 ms before the
-    // packed-row-tap kernels and 9.75 ms with the per-shape heuristic); the input-gradient convs keep the
-    // heuristic until tuned.
+    // packed-row-tap kernels and 9.75 ms with the per-shape heuristic).
     static const ConvTile kTunedFwd[14] = {{32, 16, 4, 5}, {32, 32, 3, 4}, {64, 32, 2, 4}, {64, 32, 2, 4},
                                            {64, 32, 2, 6}, {64, 32, 2, 6}, {64, 32, 2, 6}, {64, 32, 2, 6},
                                            {64, 32, 2, 6}, {64, 32, 2, 6}, {64, 32, 2, 6}, {64, 32, 2, 4},
                                            {32, 32, 2, 7}, {32, 32, 3, 4}};
     for (int i = 0; i < 14; ++i) u->tile[i] = kTunedFwd[i];
+    // Input gradients with 32 output channels at full resolution: packed row taps with resident weights, each
+    // 0.3 to 0.7% of a training pass; the gradient through the first pooling's 128 channels in two blocks of 64,
+    // 0.4%.  Together 1327 -> 1305 us at 16x128x128, 1036 -> 1016 at 8x104x144, 652 -> 643 at 4x64x64, 895 -> 878 at
+    // 2x256x256, 1113 -> 1097 at 1x512x512; the other layers gain nothing from any shape of the same K order.
+    for (int k : {0, 2, 15}) u->tile_dg[k] = {32, 32, 3, 4};
+    u->tile_dg[10] = {64, 32, 3, 1};
     cudaError_t e = cudaStreamCreateWithFlags(&u->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess)
     {
