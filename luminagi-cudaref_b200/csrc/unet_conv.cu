@@ -548,14 +548,15 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
 // walks the output tiles in a grid-stride loop.
 //   warp 0 (one lane)  TMA loads of input halos and weight blocks into a
 //                      STAGES-deep ring (full/empty mbarriers);
-//   warp 1 (one lane)  tcgen05.mma into one of two TMEM accumulators (each two
+//   warp 1             tcgen05.mma (one lane issues) into one of two TMEM accumulators (each two
 //                      rows x BN columns), committing the ring stage when its
 //                      MMAs retire and the accumulator when the tile is done;
-//   warps 2..9         the epilogue of tile i (tile_epilogue: two warps per
-//                      TMEM lane quarter, splitting the channel chunks, or the
-//                      rows of the tail) while tile i+1's loads and MMAs run;
-//                      eight warps hide the epilogue's load and store latency
-//                      behind one another.
+//   the other warps     the epilogue of tile i (tile_epilogue: two or four
+//                      warps per TMEM lane quarter, splitting the channel
+//                      chunks, or the rows of the tail) while tile i+1's loads
+//                      and MMAs run; sixteen warps hide the epilogue's load and
+//                      store latency behind one another, eight with unpooling,
+//                      whose registers do not fit sixteen.
 // Loads run ahead across tile boundaries; TMEM is allocated once per CTA.
 // The same packed weights, the same MMAs in the same order: results are
 // identical to conv3x3_tc_kernel's.
