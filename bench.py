@@ -66,9 +66,9 @@ import numpy as np  # noqa: E402
 
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # DRAM bytes (read + write) per traced ray of trace_kernel, from one ncu capture
-# of an 8-spp engine frame: 427.7 MB + 37.8 MB / 65,366,791 rays; traffic
+# of an 8-spp engine frame: 331.7 MB + 26.0 MB / 52,250,788 rays; traffic
 # scales with rays.
-TRACE_DRAM_BYTES_PER_RAY = (427703296 + 37808384) / 65366791
+TRACE_DRAM_BYTES_PER_RAY = (331665664 + 26026496) / 52250788
 # Bytes one traversal step loads from a BVH record: both 32-byte halves of a
 # 4-wide record (grid origin, steps, 24 one-byte planes, four links), or the
 # whole 64-byte 2-wide record.
@@ -78,8 +78,9 @@ RECORD_BYTES = {4: 64, 2: 64}
 CPU_ROW_STEP = 16
 # Multiply-adds per output pixel of the denoiser (14 3x3 convolutions and the 1x1 tail; ml/train.py's UNet).
 UNET_MAC_PER_PIXEL = 162240
-# Local-memory (stack and spill) bytes per traced ray of trace_kernel, from the
-# same capture: (806.4 M load + 911.3 M store sectors) x 32 B / rays.
+# Local-memory (stack and spill) bytes per traced ray of trace_kernel, from an
+# earlier capture, with the shadow rays that add exactly zero still traced:
+# (806.4 M load + 911.3 M store sectors) x 32 B / rays.
 TRACE_LOCAL_BYTES_PER_RAY = (806358764 + 911343284) * 32 / 65366791
 # Denoiser weights trained by this library on the engine scene (lumina.surrogate, the
 # 120-epoch recipe with 24 crops per image per epoch; FP16 copy of the best-validation
@@ -546,8 +547,8 @@ def main():
             "dram_bytes_per_ray": TRACE_DRAM_BYTES_PER_RAY, "kernel": "trace_kernel",
             "algorithmic_bytes_per_launch": algo_bytes, "algorithmic_bytes_per_ray": algo_bytes / rays,
             "kernel_ms": kernel_ms,
-            "limiter": "instruction issue, not memory (ncu: issue slots 71% busy at 16 of 32 lanes active, "
-                       "L1 data pipe 53%; 455 warp instructions per ray)"}
+            "limiter": "no single unit (ncu: issue slots 69% busy at 15 of 32 lanes active, waits for loads the largest "
+                       "stall, conversions 56%, L1 data pipe 55%; 421 warp instructions per ray)"}
     if TRACE_LOCAL_BYTES_PER_RAY is not None:
         roof["local_bytes_per_ray"] = TRACE_LOCAL_BYTES_PER_RAY
     line = {"metric": "Mrays/s (plain render; ms/frame alongside)", "value": value, "unit": "Mrays/s",
