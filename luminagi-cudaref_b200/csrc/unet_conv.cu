@@ -1206,6 +1206,7 @@ __global__ void pack_folded_kernel(const float* __restrict__ w, int Cout, int Ci
 __global__ void to_blocked_kernel(const float* __restrict__ x, int N, int C, int H, int W,
                                   __nv_bfloat16* __restrict__ out, int Cpad, int nb, int log1p_in, int* clear)
 {
+    begin_after_predecessors();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // over N * nb * H * W
     if (clear && i == 0) *clear = 0;
     const size_t HW = (size_t)H * W;
@@ -1507,9 +1508,8 @@ cudaError_t to_blocked_bf16(const float* x, int N, int C, int H, int W, __nv_bfl
 {
     const int nb = skip_zero_blocks ? (C + 7) / 8 : Cpad / 8;
     const size_t total = (size_t)N * nb * H * W;
-    to_blocked_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(x, N, C, H, W, out, Cpad, nb,
-                                                                         log1p_in ? 1 : 0, clear);
-    return cudaGetLastError();
+    return launch_dependent(to_blocked_kernel, (unsigned)((total + 255) / 256), 256, 0, stream, x, N, C, H, W, out, Cpad,
+                            nb, log1p_in ? 1 : 0, clear);
 }
 
 cudaError_t from_blocked_bf16(const __nv_bfloat16* in, int N, int C, int H, int W, float* out, cudaStream_t stream)

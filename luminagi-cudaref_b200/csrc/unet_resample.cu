@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "pdl.cuh"
 #include "tc_ptx.cuh"
 #include "unet_conv.cuh"
 
@@ -82,6 +83,7 @@ __device__ __forceinline__ void src_axis(int d, int n, int& i0, int& i1, float& 
 __global__ void __launch_bounds__(128) up2_kernel(const __nv_bfloat16* __restrict__ in, int N, int C, int h, int w,
                                                   __nv_bfloat16* __restrict__ out, int out_C, int coff)
 {
+    begin_after_predecessors();
     const int i = blockIdx.x * 128 + threadIdx.x;
     if (i >= w) return;
     const int H = 2 * h, W = 2 * w, CB = C >> 3;
@@ -167,8 +169,7 @@ cudaError_t bilinear_up2(const __nv_bfloat16* in, int N, int C, int h, int w, __
     if (N <= 0 || C <= 0 || h <= 0 || w <= 0 || (C % 8) || (coff % 8) || coff + C > out_C) return cudaErrorInvalidValue;
     if (2 * h > 65535 || (long long)N * (C >> 3) > 65535) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)((w + 127) / 128), (unsigned)(2 * h), (unsigned)(N * (C >> 3)));
-    up2_kernel<<<grid, 128, 0, stream>>>(in, N, C, h, w, out, out_C, coff);
-    return cudaGetLastError();
+    return launch_dependent(up2_kernel, grid, 128, 0, stream, in, N, C, h, w, out, out_C, coff);
 }
 
 cudaError_t bilinear_up2_adjoint(const __nv_bfloat16* g_hi, int N, int C, int h, int w, const __nv_bfloat16* ref,
