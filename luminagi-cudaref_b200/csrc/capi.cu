@@ -15,7 +15,6 @@
 #include "bvh.h"
 #include "common.h"
 #include "lbvh.cuh"
-#include "radix_sort.cuh"
 #include "render_tree.cuh"
 #include "scene.h"
 #include "trace.cuh"
@@ -400,14 +399,11 @@ cudaError_t post_fault(lg_renderer* r, cudaStream_t st)
 // then the stream is drained first so no copy still in flight can set it again.
 int take_fault(lg_renderer* r)
 {
-    const unsigned fault = *(volatile unsigned*)r->fault_host;
-    if (!fault) return LG_OK;
+    if (!*(volatile unsigned*)r->fault_host) return LG_OK;
     LG_TRY_CUDA(cudaStreamSynchronize(r->stream));
     LG_TRY_CUDA(cudaMemsetAsync(r->fault.p, 0, sizeof(unsigned), r->stream));
     LG_TRY_CUDA(cudaStreamSynchronize(r->stream));
     *(volatile unsigned*)r->fault_host = 0u;
-    if (fault == kRadixSortError)
-        return set_error(LG_ERR_DEVICE, "a wait of the ray sort ran out: the image is not the sorted render's");
     return set_error(LG_ERR_DEVICE,
                      "traversal stack overflow: the BVH is deeper than the %d-entry traversal stack holds, so "
                      "some subtrees were skipped and the image is incomplete",

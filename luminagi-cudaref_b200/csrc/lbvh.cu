@@ -897,7 +897,7 @@ Layout layout_for(size_t n, bool need_tmp_tris)
     L.off_tops2 = take((size_t)(chunks_for(n) + kGroup - 1) / kGroup * kTopMax * sizeof(TopNode));
     L.off_ntops = take((size_t)chunks_for(n) * 4);
     L.off_ntops2 = take((size_t)(chunks_for(n) + kGroup - 1) / kGroup * 4);
-    L.off_zero = take(256);  // bounds keys, block ticket, {node count, error}
+    L.off_zero = take(256);  // bounds keys, block ticket, node count
     L.off_sort = take(radix_sort_scratch_bytes(n));
     L.off_tmp_tris = need_tmp_tris ? take(n * sizeof(lg_triangle)) : 0;
     L.bytes = at + 256;
@@ -954,13 +954,12 @@ int lbvh_build(const lg_triangle* d_tris, int n, lg_bvh_node* d_nodes, int* n_no
     int* n_tops2 = (int*)at(L.off_ntops2);
     unsigned long long* keys = (unsigned long long*)at(L.off_zero);  // 6 bounds keys
     unsigned* ticket = (unsigned*)(keys + 6);
-    int* result = (int*)(keys + 7);  // node count, the sort's error word
-    RadixSortScratch rs = radix_sort_bind(at(L.off_sort), (size_t)n);
+    int* node_count = (int*)(keys + 7);
+    const RadixSortScratch rs = radix_sort_bind(at(L.off_sort), (size_t)n);
     const int chunks = chunks_for((size_t)n);
 
     LG_TRY_CUDA(cudaMemsetAsync(at(L.off_zero), 0, 256, stream));
     LG_TRY_CUDA(cudaMemsetAsync(rs.hist, 0, rs.zero_bytes, stream));
-    rs.error = (uint32_t*)(result + 1);
     const int grid = std::min(blocks_for((size_t)n), 148 * 8);
     LG_TRY_CUDA(launch_dependent(bounds_kernel, grid, kTB, 0, stream, d_tris, n, keys, ticket, centroids, box));
     LG_TRY_CUDA(launch_dependent(morton_kernel, std::min(grid, 148 * 4), kTB, 0, stream, centroids, n, box, codes,
@@ -971,7 +970,7 @@ int lbvh_build(const lg_triangle* d_tris, int n, lg_bvh_node* d_nodes, int* n_no
     LG_TRY_CUDA(launch_dependent(depth_kernel, chunks, kChunk, 0, stream, n, gp, skip, depth, counts, chunks));
     LG_TRY_CUDA(launch_dependent(depth_scan_kernel, kMaxDepths, kTB, 0, stream, counts, chunks, totals));
     LG_TRY_CUDA(launch_dependent(bfs_kernel, chunks, kChunk, 0, stream, n, depth, counts, chunks, totals, bfs_gap,
-                                 bfs_leaf, result));
+                                 bfs_leaf, node_count));
     lg_triangle* tris_sorted = need_tmp ? (lg_triangle*)at(L.off_tmp_tris) : d_tris_out;
     LG_TRY_CUDA(cudaFuncSetAttribute((const void*)emit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(EmitShared)));
@@ -994,11 +993,9 @@ int lbvh_build(const lg_triangle* d_tris, int n, lg_bvh_node* d_nodes, int* n_no
         LG_TRY_CUDA(cudaMemcpyAsync(d_tris_out, tris_sorted, (size_t)n * sizeof(lg_triangle),
                                     cudaMemcpyDeviceToDevice, stream));
     LG_TRY_CUDA(cudaGetLastError());
-    int got[2] = {0, 0};
-    LG_TRY_CUDA(cudaMemcpyAsync(got, result, sizeof got, cudaMemcpyDeviceToHost, stream));
+    int count = 0;
+    LG_TRY_CUDA(cudaMemcpyAsync(&count, node_count, sizeof(int), cudaMemcpyDeviceToHost, stream));
     LG_TRY_CUDA(cudaStreamSynchronize(stream));
-    if (got[1]) return set_error(LG_ERR_DEVICE, "BuildBVH: a wait of the sort ran out");
-    const int count = got[0];
     *n_nodes_host = count;
     return LG_OK;
 }

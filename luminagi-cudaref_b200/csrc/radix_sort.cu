@@ -55,7 +55,6 @@ constexpr uint32_t kAggregate = 1u << 30;  // this tile's own count of the digit
 constexpr uint32_t kInclusive = 2u << 30;  // the count of all tiles up to this one
 constexpr uint32_t kValueMask = (1u << 30) - 1u;
 constexpr int kLookBack = 8;               // predecessors read at a time
-constexpr int kPollLimit = 1 << 22;        // polls of unpublished counts before a tile gives up
 
 // Exclusive scan over the first 256 threads of one value each (every thread of the block calls it).
 __device__ __forceinline__ uint32_t digit_excl(uint32_t v, uint32_t* warp_sums)
@@ -93,7 +92,7 @@ __global__ void __launch_bounds__(kThreads) pass_kernel(const uint32_t* __restri
                                                         uint32_t* __restrict__ keys_out,
                                                         uint32_t* __restrict__ vals_out, uint32_t n, int shift,
                                                         int bits, const uint32_t* __restrict__ hist, uint32_t* state,
-                                                        uint32_t* ticket, uint32_t* error)
+                                                        uint32_t* ticket, int poll_limit)
 {
     constexpr int kTile = kThreads * kItems, kWarps = kThreads / 32;
     static_assert(kThreads >= 256, "one digit per thread");
@@ -157,7 +156,9 @@ __global__ void __launch_bounds__(kThreads) pass_kernel(const uint32_t* __restri
         uint32_t before = 0;
         if (tile > 0)
         {
-            // Add up the counts of the tiles before, nearest first, until one has its inclusive count.
+            // Add up the counts of the tiles before, nearest first, until one has its inclusive count.  Past the
+            // poll limit a count that is not there is taken from that tile's keys themselves, which no tile of this
+            // pass writes: the sort is right whatever a wait does, and what runs after it may rely on it.
             int j = (int)tile - 1, polls = 0;
             bool done = false;
             while (!done)
@@ -174,10 +175,12 @@ __global__ void __launch_bounds__(kThreads) pass_kernel(const uint32_t* __restri
                     if (v[b] >> 30 == 2) done = true;
                     --j;
                 }
-                if (!done && ++polls > kPollLimit)
+                if (!done && polls++ >= poll_limit)
                 {
-                    *error = kRadixSortError;
-                    break;
+                    polls = poll_limit;
+                    const uint32_t* of_tile = keys_in + (size_t)j * kTile;  // a whole tile: it is not the last
+                    for (int i = 0; i < kTile; ++i) before += ((of_tile[i] >> shift) & mask) == (uint32_t)tid ? 1u : 0u;
+                    done = --j < 0;
                 }
             }
             *mine = kInclusive | ((before + total) & kValueMask);
@@ -201,11 +204,8 @@ __global__ void __launch_bounds__(kThreads) pass_kernel(const uint32_t* __restri
     {
         const uint32_t k = sh.key[i];
         const uint32_t pos = sh.global_base[(k >> shift) & mask] + i;
-        if (pos < n)  // always, unless a wait ran out
-        {
-            keys_out[pos] = k;
-            vals_out[pos] = sh.val[i];
-        }
+        keys_out[pos] = k;
+        vals_out[pos] = sh.val[i];
     }
 }
 
@@ -216,7 +216,8 @@ struct PassArgs
     uint32_t n;
     int shift, bits;
     const uint32_t* hist;
-    uint32_t *state, *ticket, *error;
+    uint32_t *state, *ticket;
+    int poll_limit;
 };
 template <int kThreads, int kItems>
 cudaError_t launch_pass(const PassArgs& a, bool iota, size_t tiles, cudaStream_t st)
@@ -226,7 +227,7 @@ cudaError_t launch_pass(const PassArgs& a, bool iota, size_t tiles, cudaStream_t
     const cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     return launch_dependent(k, (unsigned)tiles, kThreads, smem, st, a.ki, a.vi, a.ko, a.vo, a.n, a.shift, a.bits, a.hist,
-                            a.state, a.ticket, a.error);
+                            a.state, a.ticket, a.poll_limit);
 }
 }  // namespace
 
@@ -246,7 +247,6 @@ RadixSortScratch radix_sort_bind(void* base, size_t n)
     p += align256(n * 4);
     s.hist = (uint32_t*)p;
     s.tickets = s.hist + kRadixMaxPasses * 256;
-    s.error = s.tickets + kRadixMaxPasses;
     p += align256(kRadixMaxPasses * 256 * 4 + 64);
     s.state = (uint32_t*)p;
     s.zero_bytes = (size_t)((char*)(s.state + kRadixMaxPasses * tiles_for(n ? n : 1) * 256) - (char*)s.hist);
@@ -280,7 +280,7 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, size_t n, int begin
     {
         const int bits = (end_bit - shift) < 8 ? (end_bit - shift) : 8;
         const PassArgs a{ki, vi, ko, vo, (uint32_t)n, shift, bits, s.hist + pass * 256,
-                         s.state + (size_t)pass * tiles * 256, s.tickets + pass, s.error};
+                         s.state + (size_t)pass * tiles * 256, s.tickets + pass, s.poll_limit};
         const bool first = iota && pass == 0;
         switch (tile_keys(n))
         {

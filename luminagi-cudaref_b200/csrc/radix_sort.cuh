@@ -15,7 +15,8 @@
 // is what the BVH build relies on for a deterministic triangle order.
 //
 // A tile waits only for tiles that started before it, so every wait ends; it is
-// bounded all the same, and a wait that ran out sets the error word.
+// bounded all the same, and a tile whose wait ran out counts the keys it waits
+// for itself.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -25,20 +26,20 @@
 namespace lg
 {
 constexpr int kRadixMaxPasses = 4;
-constexpr uint32_t kRadixSortError = 2u;  // what a wait that ran out stores in the error word
+constexpr int kRadixPollLimit = 1 << 22;  // reads of counts not yet published before a tile counts for itself
 
 struct RadixSortScratch
 {
     uint32_t* keys_alt = nullptr;
     uint32_t* vals_alt = nullptr;
     // cleared before each sort, contiguous: digit totals per pass (4 x 256), start tickets per pass (4),
-    // the error word, and per pass and tile the 256 published counts
+    // and per pass and tile the 256 published counts
     uint32_t* hist = nullptr;
     uint32_t* tickets = nullptr;
-    uint32_t* error = nullptr;  // a caller that sorts often may point it at a word of its own, which is not cleared
     uint32_t* state = nullptr;
     size_t zero_bytes = 0;  // of the cleared part, from hist on
     size_t capacity = 0;    // elements
+    int poll_limit = kRadixPollLimit;
 };
 
 // Bytes of scratch needed for n elements.
@@ -49,9 +50,7 @@ RadixSortScratch radix_sort_bind(void* base, size_t n);
 // Sorts keys/vals in place over bits [begin_bit, end_bit), n < 2^30.  Returns a
 // CUDA error.  `counted`: the cleared part of the scratch was cleared on `stream`
 // and s.hist[pass * 256 + digit] already holds the digit totals.  `iota`:
-// vals is written only, the values are the input positions.  *s.error is
-// nonzero after the sort if a wait ran out (the result is then not sorted,
-// but every access stayed in bounds).
+// vals is written only, the values are the input positions.
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
                              const RadixSortScratch& s, cudaStream_t stream, bool counted = false, bool iota = false);
 }  // namespace lg

@@ -726,8 +726,7 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
     LG_TRY_CUDA(cudaGetLastError());
     const RadixSortScratch rs = radix_sort_bind(sort_mem, (size_t)n_nodes);
     LG_TRY_CUDA(radix_sort_pairs(depth, ids, (size_t)n_nodes, 0, 8, rs, st));
-    uint32_t max_depth = 0, sort_error = 0;
-    LG_TRY_CUDA(cudaMemcpyAsync(&sort_error, rs.error, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    uint32_t max_depth = 0;
     LG_TRY_CUDA(cudaMemcpyAsync(&max_depth, depth + n_nodes - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     LG_TRY_CUDA(launch_dependent(rank_kernel, g, kTB, 0, st, ids, n_nodes, newpos));
     LG_TRY_CUDA(launch_dependent(emit_kernel, (n_nodes + kEmitNodes - 1) / kEmitNodes, kTB, 0, st, src, ids, newpos,
@@ -736,7 +735,6 @@ int build_render_tree(const lg_bvh_node* d_nodes, int n_nodes, const lg_triangle
     LG_TRY_CUDA(cudaMemcpyAsync(level_start_host, d_level_start, 257 * sizeof(int), cudaMemcpyDeviceToHost, st));
     LG_TRY_CUDA(cudaGetLastError());
     LG_TRY_CUDA(cudaStreamSynchronize(st));
-    if (sort_error) return set_error(LG_ERR_DEVICE, "render tree: a wait of the sort ran out");
     if (max_depth >= 255u) return set_error(LG_ERR_CAPACITY, "render tree: depth over 254");
     *levels = (int)max_depth + 1;
     return LG_OK;

@@ -539,8 +539,7 @@ cudaError_t launch_wavefront_frame(const DevScene& s, const DevCam& cam, const W
     slots[0] = (uint32_t*)p; p += up((size_t)n * sizeof(uint32_t));
     slots[1] = (uint32_t*)p; p += up((size_t)n * sizeof(uint32_t));
     uint32_t* rng = (uint32_t*)p; p += up((size_t)n * sizeof(uint32_t));
-    RadixSortScratch rs = radix_sort_bind(p, (size_t)n);
-    rs.error = s.fault;  // a sort's failed wait is reported as the traversals' overflows are
+    const RadixSortScratch rs = radix_sort_bind(p, (size_t)n);
     p += up(radix_sort_scratch_bytes((size_t)n));
     Staged sb;
     sb.hit = (int4*)p; p += up((size_t)n * sizeof(int4));
