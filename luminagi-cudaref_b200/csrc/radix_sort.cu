@@ -8,6 +8,8 @@
 // and 20 us.
 #include "radix_sort.cuh"
 
+#include <algorithm>
+
 #include "pdl.cuh"
 
 namespace lg
@@ -22,6 +24,8 @@ constexpr int kHistThreads = 256;
 // per SM: 15 us a pass in tiles of 8,192 there, 22 us in tiles of 2,048.
 int tile_keys(size_t n) { return n <= 148 * 1024 ? 1024 : (n <= 148 * 2048 ? 2048 : (n <= 148 * 4096 ? 4096 : 8192)); }
 size_t tiles_for(size_t n) { return (n + tile_keys(n) - 1) / tile_keys(n); }
+// Most tiles of a sort of n pairs or fewer: just below the size from which tiles are larger there are 148.
+size_t tiles_within(size_t n) { return std::max(tiles_for(n), std::min<size_t>((n + 1023) / 1024, 148)); }
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Digit totals of every pass in one read of the keys.
@@ -233,7 +237,7 @@ cudaError_t launch_pass(const PassArgs& a, bool iota, size_t tiles, cudaStream_t
 
 size_t radix_sort_scratch_bytes(size_t n)
 {
-    const size_t t = tiles_for(n ? n : 1);
+    const size_t t = tiles_within(n ? n : 1);
     return align256(n * 4) * 2 + align256(kRadixMaxPasses * 256 * 4 + 64) + kRadixMaxPasses * t * 256 * 4 + 512;
 }
 
@@ -249,7 +253,7 @@ RadixSortScratch radix_sort_bind(void* base, size_t n)
     s.tickets = s.hist + kRadixMaxPasses * 256;
     p += align256(kRadixMaxPasses * 256 * 4 + 64);
     s.state = (uint32_t*)p;
-    s.zero_bytes = (size_t)((char*)(s.state + kRadixMaxPasses * tiles_for(n ? n : 1) * 256) - (char*)s.hist);
+    s.zero_bytes = (size_t)((char*)(s.state + kRadixMaxPasses * tiles_within(n ? n : 1) * 256) - (char*)s.hist);
     s.capacity = n;
     return s;
 }
@@ -257,6 +261,7 @@ RadixSortScratch radix_sort_bind(void* base, size_t n)
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
                              const RadixSortScratch& s, cudaStream_t stream, bool counted, bool iota)
 {
+    if (n > s.capacity) return cudaErrorInvalidValue;
     if (!counted)
     {
         const cudaError_t e = cudaMemsetAsync(s.hist, 0, s.zero_bytes, stream);

@@ -42,13 +42,13 @@ struct RadixSortScratch
     int poll_limit = kRadixPollLimit;
 };
 
-// Bytes of scratch needed for n elements.
+// Bytes of scratch needed for n elements, or any fewer.
 size_t radix_sort_scratch_bytes(size_t n);
 // Carves the scratch pointers out of `base` (aligned to 256 bytes).
 RadixSortScratch radix_sort_bind(void* base, size_t n);
 
-// Sorts keys/vals in place over bits [begin_bit, end_bit), n < 2^30.  Returns a
-// CUDA error.  `counted`: the cleared part of the scratch was cleared on `stream`
+// Sorts keys/vals in place over bits [begin_bit, end_bit), n < 2^30 and at most
+// s.capacity.  Returns a CUDA error.  `counted`: the cleared part of the scratch was cleared on `stream`
 // and s.hist[pass * 256 + digit] already holds the digit totals.  `iota`:
 // vals is written only, the values are the input positions.
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,

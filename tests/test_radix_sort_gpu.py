@@ -67,3 +67,8 @@ def test_tile_shapes(n):
 @pytest.mark.parametrize("bits", [8, 30, 32])
 def test_right_without_waiting(n, bits):
     _check(n, bits, n + bits, poll_limit=0)
+
+
+@pytest.mark.parametrize("n,room", [(148 * 1024, 148 * 1024 + 1), (20500, 400001), (148 * 2048, 148 * 4096)])
+def test_fewer_pairs_than_bound_for(n, room):
+    _check(n, 30, n, bound_for=room)
