@@ -73,6 +73,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
         __nanosleep(64);
     }
 }
+// The same by a whole warp, which goes on together and with one outcome.  Lanes leave mbar_wait each on its own;
+// without the vote lane 0 could go on, free the stage and let it be filled again while another lane still polls
+// for a parity that then means a later phase, and lanes of different outcomes would part for good.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
+}
 
 // 5-D tiled TMA load into this CTA's shared memory, completing on `bar`.
 __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2,

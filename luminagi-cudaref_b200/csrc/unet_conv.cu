@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_tc_kernel(const __grid_co
     }
     __syncwarp();
     // Epilogue: every thread owns TMEM lane = pixel x0 + tid.
-    const bool got = tc::mbar_wait(done, 0);
+    const bool got = tc::mbar_wait_warp(done, 0);
     if (!got && a.err) atomicExch(a.err, 2);
     tc::tc_fence_after();
     if (got && !s_fail) tile_epilogue<BN, EPI>(a, ec, tmem, warp, tid, n, ct, x0, y0);
@@ -764,11 +764,12 @@ __global__ void __launch_bounds__(pthreads(EPI), 1) conv3x3_tc_persistent(const 
         // against 155.4 at 1x128x128.
         const bool leader = lane == 0;
         int it = 0, j = 0;
-        if (RESW && !tc::mbar_wait(wfull, 0) && leader) fail(5);
-        for (int t = blockIdx.x; t < n_tiles && !s_fail; t += gridDim.x, ++j)
+        auto failed = [&]() { return __any_sync(0xffffffffu, s_fail) != 0; };
+        if (RESW && !tc::mbar_wait_warp(wfull, 0) && leader) fail(5);
+        for (int t = blockIdx.x; t < n_tiles && !failed(); t += gridDim.x, ++j)
         {
             const int b = j & 1, v = j >> 1;
-            if (v > 0 && !tc::mbar_wait(&acc_empty[b], (uint32_t)((v - 1) & 1)))
+            if (v > 0 && !tc::mbar_wait_warp(&acc_empty[b], (uint32_t)((v - 1) & 1)))
             {
                 if (leader) fail(4);
                 break;
@@ -779,7 +780,7 @@ __global__ void __launch_bounds__(pthreads(EPI), 1) conv3x3_tc_persistent(const 
             for (int kb = 0; kb < KB; ++kb, ++it)
             {
                 const int s = it % STAGES;
-                if (!tc::mbar_wait(&full[s], (uint32_t)((it / STAGES) & 1)))
+                if (!tc::mbar_wait_warp(&full[s], (uint32_t)((it / STAGES) & 1)))
                 {
                     ok = false;
                     break;
@@ -901,7 +902,7 @@ __global__ void __launch_bounds__(pthreads(EPI), 1) conv3x3_tc_persistent(const 
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++j)
         {
             const int b = j & 1, v = j >> 1;
-            if (!tc::mbar_wait(&acc_full[b], (uint32_t)(v & 1)))
+            if (!tc::mbar_wait_warp(&acc_full[b], (uint32_t)(v & 1)))
             {
                 fail(2);
                 break;

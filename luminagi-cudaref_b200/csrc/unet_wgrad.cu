@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool have = false;
     if (steps > 0)
     {
-        const bool got = tc::mbar_wait(done, 0);
+        const bool got = tc::mbar_wait_warp(done, 0);
         if (!got && a.err) atomicExch(a.err, 4);
         tc::tc_fence_after();
         have = got && !s_fail;
