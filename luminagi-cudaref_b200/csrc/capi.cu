@@ -387,6 +387,18 @@ bool stack_safe(const lg_renderer* r)
     return (r->bvh_width == 4 ? r->stack4 : r->stack2) <= kTraceStack;
 }
 
+// Work queued on `then` from here on starts after what is on `first` by now.
+int order_streams(cudaStream_t first, cudaStream_t then)
+{
+    cudaEvent_t ev;
+    LG_TRY_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    cudaError_t e = cudaEventRecord(ev, first);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(then, ev, 0);
+    cudaEventDestroy(ev);
+    LG_TRY_CUDA(e);
+    return LG_OK;
+}
+
 // Queues a copy of the device fault word into its pinned host copy, after
 // the launches already on `st`.
 cudaError_t post_fault(lg_renderer* r, cudaStream_t st)
@@ -1155,23 +1167,9 @@ int lg_render_device(lg_renderer* r, const lg_camera* cam, const lg_render_opts*
     // An overflow in an earlier asynchronous frame is reported here.
     LG_TRY(take_fault(r));
     // Order the renderer's stream after the caller's stream.
-    if (stream)
-    {
-        cudaEvent_t ev;
-        LG_TRY_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        cudaEventRecord(ev, (cudaStream_t)stream);
-        cudaStreamWaitEvent(r->stream, ev, 0);
-        cudaEventDestroy(ev);
-    }
+    if (stream) LG_TRY(order_streams((cudaStream_t)stream, r->stream));
     LG_TRY(render_into_device(r, cam, o, nullptr));
-    if (stream)
-    {
-        cudaEvent_t ev;
-        LG_TRY_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        cudaEventRecord(ev, r->stream);
-        cudaStreamWaitEvent((cudaStream_t)stream, ev, 0);
-        cudaEventDestroy(ev);
-    }
+    if (stream) LG_TRY(order_streams(r->stream, (cudaStream_t)stream));
     else
     {
         LG_TRY_CUDA(cudaStreamSynchronize(r->stream));

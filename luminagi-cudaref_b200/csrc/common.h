@@ -20,12 +20,17 @@ static_assert(sizeof(lg_point_light) == 32, "lg_point_light layout");
 static_assert(sizeof(lg_dir_light) == 28, "lg_dir_light layout");
 }  // namespace lg
 
+// An error is reported once: it does not stay behind as the thread's last error, where the next launch's check, or
+// the caller's own, would find it.
 #define LG_TRY_CUDA(expr)                                                                          \
     do {                                                                                           \
         cudaError_t e_ = (expr);                                                                   \
         if (e_ != cudaSuccess)                                                                     \
+        {                                                                                          \
+            cudaGetLastError();                                                                    \
             return ::lg::set_error(LG_ERR_CUDA, "%s:%d: %s: %s", __FILE__, __LINE__, #expr,        \
                                    cudaGetErrorString(e_));                                        \
+        }                                                                                          \
     } while (0)
 
 #define LG_TRY(expr)                                                                               \
