@@ -76,11 +76,15 @@ def ref_available() -> bool:
     return REF_LIB.exists()
 
 
+class ReferenceMissing(RuntimeError):
+    """The reference's library has not been built here."""
+
+
 def rlib():
     global _rlib
     if _rlib is None:
         if not REF_LIB.exists():
-            raise RuntimeError(f"{REF_LIB} missing: run `make -C {HERE} ref` where the reference checkout exists")
+            raise ReferenceMissing(f"{REF_LIB} missing: run `make -C {HERE} ref` where the reference checkout exists")
         _rlib = C.CDLL(str(REF_LIB))
         _rlib.ref_scene_load.restype = C.c_void_p
         _rlib.ref_scene_load.argtypes = [C.c_char_p]
