@@ -152,7 +152,9 @@ typedef struct {
     float kernel_ms;       /* device time of the trace + tonemap launches */
     /* The rest is filled only while counting is on (lg_renderer_set_counting). */
     uint64_t closest_rays; /* closest-hit rays traced (camera + bounce) */
-    uint64_t shadow_rays;  /* shadow rays traced */
+    uint64_t shadow_rays;  /* shadow rays traced; lg_render traces none towards a point light that adds exactly zero
+                              (from one radius on), where the reference and lg_render_sorted trace them up to three
+                              radii: the same image from fewer rays */
     uint64_t node_fetches; /* 64-byte two-child BVH records read */
     uint64_t tri_tests;    /* ray/triangle tests (48 bytes of vertex data each) */
     uint64_t leaf_fetches; /* 8-byte leaf-table entries read */
