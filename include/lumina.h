@@ -401,13 +401,16 @@ int lg_unet_wait_selftest(lg_unet* u, int64_t limit_ns);
  * receives 30 (bn, kc, stages, kernel) quadruples, forward layers first.
  * The Adam state is reset.  Until then (or lg_unet_set_tiles) the forward
  * convolutions use the choice this autotuner made at batch 8, 1728x864 on
- * B200, and the input-gradient convolutions a per-shape default. */
+ * B200, and the input-gradient convolutions a per-shape default, but for 0,
+ * 2 and 15 (32 output channels at full resolution: (32, 32, 3, 4)) and 10
+ * (the first pooling's 128 channels: (64, 32, 3, 1)). */
 #define LG_UNET_TUNE_BACKWARD 1
 int lg_unet_autotune(lg_unet* u, int n, int h, int w, int flags, int32_t* tiles_out);
 /* Sets the 30 tile choices directly, in lg_unet_autotune's format; e.g. to
- * reuse a tuning result without timing.  (0, 0, 0, p) is the default shape on
- * the kernel p selects (0: one tile per CTA, 1: persistent; 2 only with an
- * explicit shape compiled for it). */
+ * reuse a tuning result without timing.  (0, 0, 0, p) is the per-shape
+ * default on the kernel p selects (0: one tile per CTA, 1: persistent; 2 only
+ * with an explicit shape compiled for it); it is not what a network starts
+ * with, see lg_unet_autotune. */
 int lg_unet_set_tiles(lg_unet* u, const int32_t* tiles);
 /* Folded upsampling (on by default): in inference passes of a network with
  * nearest upsampling, u3a, u2a and u1a read the upsampled half of their input
