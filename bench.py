@@ -78,10 +78,9 @@ RECORD_BYTES = {4: 64, 2: 64}
 CPU_ROW_STEP = 16
 # Multiply-adds per output pixel of the denoiser (14 3x3 convolutions and the 1x1 tail; ml/train.py's UNet).
 UNET_MAC_PER_PIXEL = 162240
-# Local-memory (stack and spill) bytes per traced ray of trace_kernel, from an
-# earlier capture, with the shadow rays that add exactly zero still traced:
-# (806.4 M load + 911.3 M store sectors) x 32 B / rays.
-TRACE_LOCAL_BYTES_PER_RAY = (806358764 + 911343284) * 32 / 65366791
+# Local-memory (stack and spill) bytes per traced ray of trace_kernel, from one ncu
+# capture of an 8-spp engine frame: (652.7 M load + 623.6 M store sectors) x 32 B / rays.
+TRACE_LOCAL_BYTES_PER_RAY = (652675092 + 623559182) * 32 / 52250788
 # Denoiser weights trained by this library on the engine scene (lumina.surrogate, the
 # 120-epoch recipe with 24 crops per image per epoch; FP16 copy of the best-validation
 # parameters, with the indices of the poses held out of training).
@@ -546,11 +545,9 @@ def main():
             "hbm_peak": peaks["hbm_gbs"], "hbm_frac": achieved / peaks["hbm_gbs"], "hbm_peak_source": peak_kind,
             "dram_bytes_per_ray": TRACE_DRAM_BYTES_PER_RAY, "kernel": "trace_kernel",
             "algorithmic_bytes_per_launch": algo_bytes, "algorithmic_bytes_per_ray": algo_bytes / rays,
-            "kernel_ms": kernel_ms,
+            "kernel_ms": kernel_ms, "local_bytes_per_ray": TRACE_LOCAL_BYTES_PER_RAY,
             "limiter": "no single unit (ncu: issue slots 69% busy at 15 of 32 lanes active, waits for loads the largest "
                        "stall, conversions 56%, L1 data pipe 55%; 421 warp instructions per ray)"}
-    if TRACE_LOCAL_BYTES_PER_RAY is not None:
-        roof["local_bytes_per_ray"] = TRACE_LOCAL_BYTES_PER_RAY
     line = {"metric": "Mrays/s (plain render; ms/frame alongside)", "value": value, "unit": "Mrays/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
