@@ -761,7 +761,9 @@ __global__ void __launch_bounds__(pthreads(EPI), 1) conv3x3_tc_persistent(const 
         // against lane 0 alone building each one: 622 -> 611 us a pass at 1x864x1728, 550 -> 541 (HDR, 1x720x1280),
         // 4.71 -> 4.66 ms at 8x864x1728, 157.2 -> 155.5 us at 1x128x128, 178.6 -> 178.6 at 1x256x512 with 12
         // channels.  With the offsets but lane 0 alone in the loops: 4.43 ms against 4.38 at 8x864x1728, 157.6 us
-        // against 155.4 at 1x128x128.
+        // against 155.4 at 1x128x128.  (Only times of one comparison belong together: a pass at 8x864x1728 takes
+        // 4.10 ms for the first ten at 1,965 MHz, 4.39 over thirty, and 4.67 over a thousand at 1,650 MHz, under the
+        // power cap.)
         const bool leader = lane == 0;
         int it = 0, j = 0;
         auto failed = [&]() { return __any_sync(0xffffffffu, s_fail) != 0; };
@@ -1197,9 +1199,6 @@ __global__ void pack_folded_kernel(const float* __restrict__ w, int Cout, int Ci
     }
     out[i] = __float2bfloat16_rn(v);
 }
-
-// Input-gradient weights: output (ct, kb, tap, kc8, j, e) of a conv with
-// Cin' = Cout (forward) and Cout' = ci_cnt reads w[co = ci'][ci_lo + co'][2-ky][2-kx].
 
 // One thread per (image, 8-channel block, pixel) of the first nb blocks:
 // reads the block's channels from their NCHW planes (consecutive threads,
