@@ -355,6 +355,10 @@ def main():
             return
         sys.path.insert(0, str(ROOT / "oracle"))
         import oracle as O
+        if not O.ref_available():
+            print(json.dumps({"impl": "reference", "unavailable": "the reference's library (oracle/_ref/libref.so) is not "
+                              "built here: its sources are absent"}))
+            return
         nodes, tris = O.ref_build_bvh(scene.tris)  # the reference's own BuildBVH
         rays = sample_rays(scene, nodes, tris, args.spp, args.bounces, args.cpu_row_step)
         vals = []
